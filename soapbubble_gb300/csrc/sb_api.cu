@@ -566,6 +566,9 @@ int sb_create(const sb_params* p, sb_bubble** out) {
     f.dmass = F32(a.dmass); f.cE = F32(a.cE); f.cS = F32(a.cS); f.rhs = F32(a.rhs); f.r0 = F32(a.r0);
     f.x = F32(a.x); f.dx = F32(a.dx); f.r = F32(a.r); f.z = F32(a.z); f.z1 = F32(a.z1);
     f.p = F32(a.p); f.q = F32(a.q);
+    // z, z1, p, q follow one another without gaps: N * 4 bytes is a multiple
+    // of the 256 that the arena rounds to (N = 2 nTheta^2, nTheta >= 8)
+    f.eta_near = (float2*)f.z; f.eta_far = f.p; f.changes = (float4*)f.z;
     f.xff = (float2*)(A + a.xff);
     f.pcr = (float*)(A + a.pcr);
     f.pcr_levels = (int*)(A + a.pcr_levels);
@@ -654,6 +657,7 @@ int sb_create(const sb_params* p, sb_bubble** out) {
         d.ph = b->ph;
         d.f = f;
         d.cur = 0;
+        d.chains = uses_chains(g, b->storage) ? 1 : 0;
         const int roff[2] = {0, g.nT};
         SbBubbleDesc** self_list = (SbBubbleDesc**)(A + a.self_list);
         e = cudaMemcpy(f.self, &d, sizeof(d), cudaMemcpyHostToDevice);
@@ -667,6 +671,7 @@ int sb_create(const sb_params* p, sb_bubble** out) {
             for (int c = 0; c < g.N; c += kTileSizes[k]) tl.push_back(make_int2(0, c));
             P.tiles[k] = (const int2*)(A + a.tiles[k]);
             P.ntiles[k] = (int)tl.size();
+            P.nchain[k] = d.chains ? P.ntiles[k] : 0;
             e = cudaMemcpy((void*)P.tiles[k], tl.data(), sizeof(int2) * tl.size(), cudaMemcpyHostToDevice);
         }
         for (int st = 0; st < STAGE_COUNT; ++st) P.sel[st] = 1;
@@ -1549,8 +1554,13 @@ int sb_batch_create(sb_bubble* const* bubbles, int n, sb_batch** out) {
     // tiles for the three tile sizes
     std::vector<int2> tiles[3];
     for (int s = 0; s < 3; ++s)
-        for (int k = 0; k < n; ++k)
-            for (int c = 0; c < B->m[k]->g.N; c += kTileSizes[s]) tiles[s].push_back(make_int2(k, c));
+        for (int chains = 1; chains >= 0; --chains) {  // the chain kernels' members first
+            for (int k = 0; k < n; ++k)
+                if (B->m[k]->desc.chains == chains)
+                    for (int c = 0; c < B->m[k]->g.N; c += kTileSizes[s])
+                        tiles[s].push_back(make_int2(k, c));
+            if (chains) P.nchain[s] = (int)tiles[s].size();
+        }
     Layout L;
     const size_t o_desc = L.take(sizeof(SbBubbleDesc*) * n);
     size_t o_tiles[3];

@@ -97,7 +97,7 @@ __device__ __forceinline__ float bilerp(float f00, float f01, float f10, float f
 
 // Grid position of the point C + d.  Points past a pole come back with the
 // base column shifted by nTheta (azimuth + pi) so the float offset stays small.
-__device__ SB_CONV_INLINE Pos pos_from_disp(Frame F, f3 d, float invh, int nT) {
+static __device__ SB_CONV_INLINE Pos pos_from_disp(Frame F, f3 d, float invh, int nT) {
     const float Px = F.s0 + d.x, Py = d.y, Pz = F.c0 + d.z;
     const float rho = sqrtf(Px * Px + Py * Py);
     const float den = rho + F.s0;
@@ -121,7 +121,7 @@ __device__ SB_CONV_INLINE Pos pos_from_disp(Frame F, f3 d, float invh, int nT) {
 // departure points of field samples and of map lookups whose result is not
 // stored): the same formulas with the quotients taken by __fdividef, which
 // places the point within ~1e-6 of a cell.
-__device__ SB_CONV_INLINE Pos pos_from_disp_fast(Frame F, f3 d, float invh, int nT) {
+static __device__ SB_CONV_INLINE Pos pos_from_disp_fast(Frame F, f3 d, float invh, int nT) {
     const float Px = F.s0 + d.x, Py = d.y, Pz = F.c0 + d.z;
     const float rho = sqrtf(Px * Px + Py * Py);
     const float den = rho + F.s0;
@@ -152,7 +152,7 @@ __device__ __forceinline__ float dist_from_disp(f3 d, float invh) {
 // slerp(A, B, a) = sin((1-a)W)/sin W A + sin(aW)/sin W B, written so that
 // nearby points keep full precision: slerp - C = cA dA + cB dB + k C with
 // k = cA + cB - 1 = 2 sin((1-a)W/2) sin(aW/2) / cos(W/2).
-__device__ __noinline__ f3 slerp_disp_far(float s0, float c0, f3 dA, f3 dB, float a) {
+static __device__ __noinline__ f3 slerp_disp_far(float s0, float c0, f3 dA, f3 dB, float a) {
     const f3 e = dB - dA;
     const float W = farc_of_chord(len3(e));
     const float b = 1.0f - a;

@@ -14,11 +14,11 @@ namespace sb {
 // Cold paths: the library functions for arguments outside the fast
 // intervals, kept out of line so that the hot loops stay small in the
 // instruction cache.
-__device__ __noinline__ void slow_sincos(float x, float* s, float* c) { sincosf(x, s, c); }
-__device__ __noinline__ float slow_sinc(float x) { return sinf(x) / x; }
-__device__ __noinline__ float slow_cos(float x) { return cosf(x); }
-__device__ __noinline__ float slow_arc(float x) { return 2.0f * asinf(fminf(x, 1.0f)); }
-__device__ __noinline__ float slow_atan2(float y, float x) { return atan2f(y, x); }
+static __device__ __noinline__ void slow_sincos(float x, float* s, float* c) { sincosf(x, s, c); }
+static __device__ __noinline__ float slow_sinc(float x) { return sinf(x) / x; }
+static __device__ __noinline__ float slow_cos(float x) { return cosf(x); }
+static __device__ __noinline__ float slow_arc(float x) { return 2.0f * asinf(fminf(x, 1.0f)); }
+static __device__ __noinline__ float slow_atan2(float y, float x) { return atan2f(y, x); }
 
 // sin and cos; Taylor to x^3 / x^4 on |x| <= 1/32 (the usual half-angle of
 // a few cells; relative truncation < 1e-8), to x^7 / x^8 on |x| <= 0.2

@@ -66,6 +66,11 @@ struct SbFields {
     // analytically; rhs = b (for the norm only)
     float *dmass, *cE, *cS, *rhs, *r0;
     float *x, *dx, *r, *z, *z1, *p, *q;            // solver vectors
+    // sampled together by the chain kernels; they lie over z, z1, p
+    // and q, which are dead outside the solve
+    float2* eta_near;                              // (init, delta) of the thickness (z, z1)
+    float* eta_far;                                // initL + deltaL of the thickness (p)
+    float4* changes;                               // (d_eta, d_gam, eta, gam) after the solve (z .. q)
     float2 *xff;                                   // mixed-precision iterate (float-float)
     float *pcr;                                    // phi-line factors, one blob per row
     int *pcr_levels;                               // reduction levels per row
@@ -90,8 +95,13 @@ struct SbBubbleDesc {
     int halted;        // 1: the kernels leave this bubble untouched (set by k_flip)
     int halt_on_fail;  // 1: a step whose solve missed its tolerance halts the bubble
                        // (the frame loop of sb_run stops at that step, as Bubble::run)
-    int pad;
+    int chains;        // 1: the chain kernels serve this bubble (uses_chains)
 };
+
+// Whether the chain kernels (sb_step.cu) serve a bubble.
+inline bool uses_chains(const SbGrid& g, int storage) {
+    return storage == kStoreF32 && g.nT <= 512;
+}
 
 // Preconditioner of the implicit solve: the exact phi-line blocks B alone,
 // with the Neumann term B^-1 C B^-1 added (C: the theta couplings), or
@@ -188,8 +198,10 @@ extern const int kTileSizes[3];
 struct SbStepPlan {
     SbBubbleDesc* const* descs;  // [nb]
     int nb;
-    const int2* tiles[3];        // (bubble, first cell) of every tile, per tile size
+    const int2* tiles[3];        // (bubble, first cell) of every tile, per tile size; the tiles
+                                 // of bubbles that the chain kernels serve come first
     int ntiles[3];
+    int nchain[3];               // the first of them, whose bubbles the chain kernels serve
     int sel[STAGE_COUNT];        // tile size (index into kTileSizes) of every stage
     SbSolveSet set;              // every bubble's implicit system
     int maxNP;                   // widest grid of the set
@@ -203,6 +215,9 @@ struct SbStepPlan {
 cudaError_t prepare_plan(const SbStepPlan& P);
 // One stage of a step, the map-parity flip that ends a step, or the whole step.
 cudaError_t launch_plan_stage(const SbStepPlan& P, int stage, cudaStream_t s);
+// A map, velocity, thickness or accumulation stage of the members that the
+// chain kernels serve (sb_chain.cu).
+void launch_chain_stage(const SbStepPlan& P, int stage, cudaStream_t s);
 cudaError_t launch_plan_flip(const SbStepPlan& P, cudaStream_t s);
 cudaError_t launch_plan_step(const SbStepPlan& P, cudaStream_t s);
 // Self-test of the bounded grid barrier on a bubble's barrier word (`blocks`

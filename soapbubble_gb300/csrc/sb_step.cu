@@ -20,7 +20,7 @@
 // van der Waals is identically zero in the reference (W1 = W2 = 0,
 // bubble.cu:2633-2638) and is folded out.
 
-#include "sb_device.cuh"
+#include "sb_cells.cuh"
 #include "sb_internal.h"
 #include "sb_scale.cuh"
 #include "sb_sync.cuh"
@@ -31,38 +31,11 @@ namespace {
 
 constexpr int kBlock = 128;
 
-__constant__ float kW5[5] = {0.125f, 0.125f, 0.125f, 0.125f, 0.5f};
-
-__device__ __forceinline__ Frame face_frame_uphi(const SbGrid& g, int i, int j) {
-    Frame F;
-    F.bi = i; F.bj = j; F.fi = 0.5f; F.fj = -0.5f;
-    F.s0 = g.sin_c[i]; F.c0 = g.cos_c[i];
-    F.s0lo = 0.0f; F.c0lo = 0.0f;
-    return F;
-}
-
-__device__ __forceinline__ Frame face_frame_utheta(const SbGrid& g, int i, int j) {
-    Frame F;
-    F.bi = i + 1; F.bj = j; F.fi = 0.0f; F.fj = 0.0f;
-    F.s0 = g.sin_e[i + 1]; F.c0 = g.cos_e[i + 1];
-    F.s0lo = 0.0f; F.c0lo = 0.0f;
-    return F;
-}
-
-__device__ __forceinline__ Pos pos_of(const Frame& F, const Trace& T, const SbGrid& g) {
-    return T.moved ? pos_from_disp(F, T.d, g.invh, g.nT) : frame_pos(F, 0.0f, 0.0f);
-}
-
 // ---------------------------------------------------------------------------
 template <class T>
 __device__ __forceinline__ void advect_maps_cell(const SbGrid& g, const SbPhys& ph, const SbFields& f, int cur,
                                           int idx) {
     (void)cur;
-    if (idx == 0) {
-        f.stats->distortion_bits = 0u;
-        f.stats->reinit = 0;
-        f.stats->broken_cells = 0;
-    }
     const int i = idx >> g.logP, j = idx & g.maskP;
     const float dt = f.step->dt;
     const Frame F = cell_frame(g, i, j);
@@ -91,59 +64,14 @@ __device__ __forceinline__ void advect_maps_cell(const SbGrid& g, const SbPhys& 
         f.gam_adv[idx] = gather_s<T>(f.gam, sstencil_of(g, cb), ph.base_gam);
     }
 
-    // air flow = initial wind + corridor(t); NaN -> 0
-    const float wg = f.step->windg;
-    float ua = f.uair_init[idx] + wg * f.corr_u[idx];
-    f.uair[idx] = isnan(ua) ? 0.0f : ua;
-    if (i < g.nT - 1) {
-        float va = f.vair_init[idx] + wg * f.corr_v[idx];
-        f.vair[idx] = isnan(va) ? 0.0f : va;
-    }
-}
-
-// Velocity self-advection with parallel transport (RUNGE_KUTTA path).
-__device__ __forceinline__ float advect_velocity(const SbGrid& g, const float* __restrict__ uth,
-                                                 const float* __restrict__ uph, const Frame& F,
-                                                 float gt, float gp, float dt, bool outPhi,
-                                                 bool rk2) {
-    const f3 w = {F.s0, 0.0f, F.c0};
-    // a zero or NaN speed stops the trace; the reference then writes that
-    // speed (bubble.cu:689-692, 727-730)
-    const Trace T = trace_gc<true>(g, uth, uph, F, gt, gp, dt, rk2);
-    if (!T.moved) return T.fail;
-    const f3 P = w + T.d;
-    const Pos qp = pos_from_disp_fast(F, T.d, g.invh, g.nT);
-    float pt, pp;
-    velocity_at(g, uth, uph, qp, pt, pp);
-    f3 beth, beph;
-    basis_at(P, beth, beph);
-    const f3 pu = pt * beth + pp * beph;
-    const f3 uCircleP = T.cd * T.u_ - T.sd * w;
-    const f3 vCircleP = cross3(P, uCircleP);
-    const float a = dot3(pu, vCircleP);
-    const float b = dot3(pu, uCircleP);
-    const f3 pu2 = b * T.u_ + a * T.v_;
-    if (outPhi) return pu2.y;                       // e_phi = (0, 1, 0)
-    return pu2.x * F.c0 - pu2.z * F.s0;             // e_theta = (c0, 0, -s0)
+    step_start(g, f, idx);
 }
 
 __device__ __forceinline__ void velocity_cell(const SbGrid& g, const SbPhys& ph, const SbFields& f, int cur,
                                           int idx) {
     (void)cur;
-    const int i = idx >> g.logP, j = idx & g.maskP;
-    const float dt = f.step->dt;
-    {
-        const Frame F = face_frame_uphi(g, i, j);
-        const float gp = f.uph[idx];
-        const float gt = sample_utheta(g, f.uth, frame_pos(F, 0.0f, 0.0f));
-        f.uph_adv[idx] = advect_velocity(g, f.uth, f.uph, F, gt, gp, dt, true, !ph.single_step);
-    }
-    if (i < g.nT - 1) {
-        const Frame F = face_frame_utheta(g, i, j);
-        const float gt = f.uth[idx];
-        const float gp = sample_uphi(g, f.uph, frame_pos(F, 0.0f, 0.0f));
-        f.uth_adv[idx] = advect_velocity(g, f.uth, f.uph, F, gt, gp, dt, false, !ph.single_step);
-    }
+    f.uph_adv[idx] = velocity_uphi(g, ph, f, idx);
+    if ((idx >> g.logP) < g.nT - 1) f.uth_adv[idx] = velocity_utheta(g, ph, f, idx);
 }
 
 // BIMOCQ thickness: compose the new backward map with the previous one and
@@ -788,7 +716,7 @@ __device__ __forceinline__ float gnew_diff_v(float xa, float2 da, float ga, floa
 // does post_cell's operations.
 template <class T>
 __device__ __forceinline__ void post_quad(const SbGrid& g, const SbPhys& ph, const SbFields& f,
-                                          int idx) {
+                                          int idx, int chains) {
     const int i = idx >> g.logP, j = idx & g.maskP;
     const int nP = g.nP;
     const float invDt = f.step->invDt, evapDt = f.step->evapDt;
@@ -864,16 +792,17 @@ __device__ __forceinline__ void post_quad(const SbGrid& g, const SbPhys& ph, con
         }
     }
     st4_s<T>(f.gam, idx, oG, ph.base_gam);
-    st4(f.d_gam + idx, oDG);
     st4_s<T>(f.eta, idx, oE, ph.base_eta);
-    st4(f.d_eta + idx, oDE);
+    if (chains) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            f.changes[idx + k] = make_float4(oDE[k], oDG[k], oE[k], oG[k]);
+    } else {
+        st4(f.d_gam + idx, oDG);
+        st4(f.d_eta + idx, oDE);
+    }
     st4(f.uph + idx, oU);
     if (hasS) st4(f.uth + idx, oV);
-}
-
-__device__ __forceinline__ float warp_max(float v) {
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
 }
 
 // BIMOCQ change accumulation through the forward map, fused with the
@@ -938,18 +867,6 @@ __device__ __forceinline__ void block_max_distortion(float dist, SbDevStats* st)
 // the cells tiles[b] = (bubble, first cell) .. + blockDim.x - 1 (a tile never
 // straddles two bubbles).  One bubble stepped alone and inside a batch runs
 // the same kernels on the same descriptor.
-// The block's bubble descriptor is copied to shared memory first, so the
-// cell code reads grid constants and array pointers from there.
-__device__ __forceinline__ const SbBubbleDesc& stage_tile_desc(SbBubbleDesc* const* descs, int b,
-                                                               SbBubbleDesc* s_d) {
-    constexpr int kWords = (int)(sizeof(SbBubbleDesc) / 4);
-    const int* src = reinterpret_cast<const int*>(descs[b]);
-    int* dst = reinterpret_cast<int*>(s_d);
-    for (int k = threadIdx.x; k < kWords; k += blockDim.x) dst[k] = src[k];
-    __syncthreads();
-    return *s_d;
-}
-
 // Kernels whose cells touch the stored thickness / surfactant fields are
 // instantiated per storage type T (float or __nv_bfloat16); a plan launches
 // the instantiation of its bubbles' storage.
@@ -1009,6 +926,9 @@ template <class T, bool VISC>
 __global__ void __launch_bounds__(256) k_post(SbBubbleDesc* const* __restrict__ descs,
                                               const int2* __restrict__ tiles) {
     SB_CELL_KERNEL_BODY(post_cell<T, VISC>)
+    if (d.chains && idx < d.g.N)  // what the accumulation's chains sample, in one word
+        d.f.changes[idx] = make_float4(d.f.d_eta[idx], d.f.d_gam[idx], ld_s<T>(d.f.eta, idx, 0.0f),
+                                       ld_s<T>(d.f.gam, idx, 0.0f));
 }
 
 // The non-viscous post-solve update, four cells per thread (a tile of n
@@ -1021,7 +941,7 @@ __global__ void __launch_bounds__(64) k_post4(SbBubbleDesc* const* __restrict__ 
     const SbBubbleDesc& d = stage_tile_desc(descs, t.x, &s_d);
     if (d.halted) return;
     const int idx = t.y + 4 * threadIdx.x;
-    if (idx < d.g.N) post_quad<T>(d.g, d.ph, d.f, idx);
+    if (idx < d.g.N) post_quad<T>(d.g, d.ph, d.f, idx, d.chains);
 }
 
 // k_accum is held to 64 registers per thread (a few spilled values): the
@@ -1256,15 +1176,23 @@ cudaError_t launch_plan_stage(const SbStepPlan& P, int stage, cudaStream_t s) {
     SbBubbleDesc* const* d = P.descs;
     const int2* t = P.tiles[k];
     const bool bf = P.storage == kStoreBF16;
+    // the tiles of the members the chain kernels serve come first
+    const int nc = P.nchain[k], nr = n - nc;
+    const int2* tr = t + nc;
     switch (stage) {
         case STAGE_MAPS:
-            if (bf) k_advect_maps<__nv_bfloat16><<<n, block, 0, s>>>(d, t);
-            else k_advect_maps<float><<<n, block, 0, s>>>(d, t);
+            if (nc) launch_chain_stage(P, stage, s);
+            if (nr && bf) k_advect_maps<__nv_bfloat16><<<nr, block, 0, s>>>(d, tr);
+            else if (nr) k_advect_maps<float><<<nr, block, 0, s>>>(d, tr);
             break;
-        case STAGE_VELOCITY: k_velocity<<<n, block, 0, s>>>(d, t); break;
+        case STAGE_VELOCITY:
+            if (nc) launch_chain_stage(P, stage, s);
+            if (nr) k_velocity<<<nr, block, 0, s>>>(d, tr);
+            break;
         case STAGE_BIMOCQ:
-            if (bf) k_bimocq<__nv_bfloat16><<<n, block, 0, s>>>(d, t);
-            else k_bimocq<float><<<n, block, 0, s>>>(d, t);
+            if (nc) launch_chain_stage(P, stage, s);
+            if (nr && bf) k_bimocq<__nv_bfloat16><<<nr, block, 0, s>>>(d, tr);
+            else if (nr) k_bimocq<float><<<nr, block, 0, s>>>(d, tr);
             break;
         case STAGE_ASSEMBLE:
             if (P.viscous) k_assemble<true><<<n, block, 0, s>>>(d, t);
@@ -1283,8 +1211,9 @@ cudaError_t launch_plan_stage(const SbStepPlan& P, int stage, cudaStream_t s) {
             }
             break;
         case STAGE_ACCUM:
-            if (bf) k_accum<__nv_bfloat16><<<n, block, 0, s>>>(d, t);
-            else k_accum<float><<<n, block, 0, s>>>(d, t);
+            if (nc) launch_chain_stage(P, stage, s);
+            if (nr && bf) k_accum<__nv_bfloat16><<<nr, block, 0, s>>>(d, tr);
+            else if (nr) k_accum<float><<<nr, block, 0, s>>>(d, tr);
             break;
         case STAGE_REINIT: {
             // the re-initialisation works on kBlock-cell tiles
