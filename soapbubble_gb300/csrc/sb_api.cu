@@ -86,6 +86,7 @@ struct sb_bubble {
     long long steps = 0;
     double last_dt = -1, last_t = -1e300;
     SbStepParams* h_step = nullptr;  // pinned
+    SbDevStats* h_stats = nullptr;   // pinned (the same allocation)
     long long launches = 0;          // kernels launched by this handle
     cudaEvent_t ev[STAGE_COUNT + 1] = {};
     SbStepPlan plan{};                 // this bubble as a set of one
@@ -334,12 +335,9 @@ float4 map_entry_from_abs(int i, int j, int nT, double th, double ph) {
     return make_float4((float)(X - std::sin(t0)), (float)Y, (float)(Z - std::cos(t0)), 0.0f);
 }
 
-// Writes the per-step scalars into the pinned slot and copies them to the
-// device on `stream`; the caller makes sure no earlier copy of the slot is
-// still in flight.
-int write_step_params(sb_bubble* b, double t, double dt_s, cudaStream_t stream) {
+// The per-step scalars of frame time t and step dt_s.
+void step_params(const sb_bubble* b, double t, double dt_s, SbStepParams* s) {
     const double dtn = dt_s * 1.0 / b->params.radius;  // dt U / r with U = 1
-    SbStepParams* s = b->h_step;
     s->dt = (float)dtn;
     s->invDt = (float)(1.0 / dtn);
     s->windg = (float)(3.0 - std::fabs(t - 3.0));
@@ -347,7 +345,14 @@ int write_step_params(sb_bubble* b, double t, double dt_s, cudaStream_t stream) 
     s->mixB = (float)(1.0 - t / 12.0);
     s->evapDt = (float)((double)b->ph.evap * dtn);
     s->pad[0] = s->pad[1] = 0.f;
-    SB_CHECK(cudaMemcpyAsync(b->f.step, s, sizeof(SbStepParams), cudaMemcpyHostToDevice, stream));
+}
+
+// Writes them into the pinned slot and copies them to the device; the caller
+// makes sure no earlier copy of the slot is still in flight.
+int write_step_params(sb_bubble* b, double t, double dt_s) {
+    step_params(b, t, dt_s, b->h_step);
+    SB_CHECK(cudaMemcpyAsync(b->f.step, b->h_step, sizeof(SbStepParams), cudaMemcpyHostToDevice,
+                             b->stream));
     b->last_dt = dt_s;
     b->last_t = t;
     return SB_OK;
@@ -356,7 +361,7 @@ int write_step_params(sb_bubble* b, double t, double dt_s, cudaStream_t stream) 
 int set_step_params(sb_bubble* b, double t, double dt_s) {
     if (dt_s == b->last_dt && t == b->last_t) return SB_OK;
     SB_CHECK(cudaStreamSynchronize(b->stream));  // the pinned slot may be in flight
-    return write_step_params(b, t, dt_s, b->stream);
+    return write_step_params(b, t, dt_s);
 }
 
 // The next solve starts from dx = 0: the state it would warm-start from has
@@ -371,25 +376,36 @@ bool state_field(sb_field w) {
     return !(w == SB_UAIR_INIT || w == SB_VAIR_INIT || w == SB_UAIR || w == SB_VAIR);
 }
 
-int reset_bimocq(sb_bubble* b) {
-    const size_t N = (size_t)b->g.N * scalar_bytes(b->storage), N4 = (size_t)b->g.N * 4;
-    SbFields& f = b->f;
-    SB_CHECK(cudaMemcpyAsync(f.eta_init, f.eta, N, cudaMemcpyDeviceToDevice, b->stream));
-    SB_CHECK(cudaMemcpyAsync(f.eta_initL, f.eta, N, cudaMemcpyDeviceToDevice, b->stream));
-    SB_CHECK(cudaMemcpyAsync(f.gam_init, f.gam, N, cudaMemcpyDeviceToDevice, b->stream));
-    SB_CHECK(cudaMemcpyAsync(f.gam_initL, f.gam, N, cudaMemcpyDeviceToDevice, b->stream));
-    SB_CHECK(cudaMemsetAsync(f.eta_delta, 0, N4, b->stream));
-    SB_CHECK(cudaMemsetAsync(f.eta_deltaL, 0, N4, b->stream));
-    SB_CHECK(cudaMemsetAsync(f.gam_delta, 0, N4, b->stream));
-    SB_CHECK(cudaMemsetAsync(f.gam_deltaL, 0, N4, b->stream));
-    SB_CHECK(launch_reset_maps(b->g, b->f, b->stream));
-    return invalidate_warm_start(b, b->stream);
+// Device buffers for uploaded FP64 arrays (8 bytes a cell): the per-step
+// increments and errors and the solver's vectors, which only live inside a
+// step, while uploads run between steps on the bubble's stream.  The arrays
+// of a pair follow one another in the arena without a gap.
+double* f64_buffer(sb_bubble* b, int k) {
+    float* const at[4] = {b->f.d_eta, b->f.err_eta, b->f.z, b->f.p};
+    return (double*)at[k];
+}
+
+// Uploads arrive in FP64 and are rounded on the device: the host's loops over
+// them took 0.25 ms of a 512 x 1024 field's 0.3, a page-locked or pageable
+// copy of the doubles takes 0.035 and the kernel 0.01.
+int copy_f64(sb_bubble* b, int k, const double* src, size_t n) {
+    SB_CHECK(cudaMemcpyAsync(f64_buffer(b, k), src, n * sizeof(double), cudaMemcpyHostToDevice, b->stream));
+    return SB_OK;
+}
+
+// BIMOCQ buffers and maps restarted from the bubble's state.
+int reset_bimocq(sb_bubble* b, const SbRestart& src = {}) {
+    SB_CHECK(launch_restart(b->g, b->f, src, b->ph, b->storage, b->stream));
+    b->launches += 1;
+    return SB_OK;
 }
 
 int upload_f32(sb_bubble* b, float* dst, const double* src, size_t n) {
-    std::vector<float> tmp(n);
-    for (size_t i = 0; i < n; ++i) tmp[i] = (float)src[i];
-    SB_CHECK(cudaMemcpyAsync(dst, tmp.data(), n * sizeof(float), cudaMemcpyHostToDevice, b->stream));
+    int rc = copy_f64(b, 0, src, n);
+    if (rc != SB_OK) return rc;
+    SB_CHECK(launch_store_f64(reinterpret_cast<SbScalar*>(dst), f64_buffer(b, 0), (int)n, 0.0f, kStoreF32,
+                              b->stream));
+    b->launches += 1;
     SB_CHECK(cudaStreamSynchronize(b->stream));
     return SB_OK;
 }
@@ -446,19 +462,18 @@ int set_base(sb_bubble* b, bool gamma, const double* v, size_t n) {
 }
 
 int upload_scalar(sb_bubble* b, SbScalar* dst, const double* src, size_t n) {
-    std::vector<float> tmp(n);
-    for (size_t i = 0; i < n; ++i) tmp[i] = (float)src[i];
-    SB_CHECK(cudaMemcpyAsync(staging(b), tmp.data(), n * sizeof(float), cudaMemcpyHostToDevice,
-                             b->stream));
-    int rc = store_from_staging(b, dst, n);
+    int rc = copy_f64(b, 0, src, n);
     if (rc != SB_OK) return rc;
+    SB_CHECK(launch_store_f64(dst, f64_buffer(b, 0), (int)n, base_of(b, dst), b->storage, b->stream));
+    b->launches += 1;
     SB_CHECK(cudaStreamSynchronize(b->stream));
     return SB_OK;
 }
 
 int fill_const(sb_bubble* b, SbScalar* dst, size_t n, float v) {
-    std::vector<double> tmp(n, (double)v);
-    return upload_scalar(b, dst, tmp.data(), n);
+    SB_CHECK(launch_fill(dst, v, (int)n, base_of(b, dst), b->storage, b->stream));
+    b->launches += 1;
+    return SB_OK;
 }
 
 }  // namespace
@@ -532,12 +547,14 @@ int sb_create(const sb_params* p, sb_bubble** out) {
     ArenaPlan a = plan_arena(g, p->storage);
     cudaError_t e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaMalloc((void**)&b->arena, a.L.bytes);
-    if (e == cudaSuccess) e = cudaMallocHost((void**)&b->h_step, sizeof(SbStepParams));
+    if (e == cudaSuccess) e = cudaMallocHost((void**)&b->h_step, 64 + sizeof(SbDevStats));
     if (e != cudaSuccess) {
         int r = cuda_fail(e, "sb_create allocation");
         sb_destroy(b);
         return r;
     }
+    static_assert(sizeof(SbStepParams) <= 64, "the statistics follow the step scalars");
+    b->h_stats = (SbDevStats*)((char*)b->h_step + 64);
     b->arena_bytes = a.L.bytes;
     e = cudaMemset(b->arena, 0, a.L.bytes);
     if (e != cudaSuccess) { int r = cuda_fail(e, "memset"); sb_destroy(b); return r; }
@@ -903,15 +920,19 @@ int sb_upload_fields(sb_bubble* b, const double* eta, const double* gamma, const
     SB_CHECK(cudaSetDevice(b->device));
     const size_t N = (size_t)b->g.N, Nv = (size_t)b->g.Nv;
     int rc = SB_OK;
-    if (eta && rc == SB_OK) rc = set_base(b, false, eta, N);
-    if (eta && rc == SB_OK) rc = upload_scalar(b, b->f.eta, eta, N);
-    if (gamma && rc == SB_OK) rc = set_base(b, true, gamma, N);
-    if (gamma && rc == SB_OK) rc = upload_scalar(b, b->f.gam, gamma, N);
-    if (u_theta && rc == SB_OK) rc = upload_f32(b, b->f.uth, u_theta, Nv);
-    if (u_phi && rc == SB_OK) rc = upload_f32(b, b->f.uph, u_phi, N);
     if (uair_init && rc == SB_OK) rc = upload_f32(b, b->f.uair_init, uair_init, N);
     if (vair_init && rc == SB_OK) rc = upload_f32(b, b->f.vair_init, vair_init, Nv);
-    if (rc == SB_OK) rc = reset_bimocq(b);
+    if (eta && rc == SB_OK) rc = set_base(b, false, eta, N);
+    if (gamma && rc == SB_OK) rc = set_base(b, true, gamma, N);
+    SbRestart src{};
+    const struct { const double* from; size_t n; const double** to; } in[4] = {
+        {eta, N, &src.eta}, {gamma, N, &src.gamma}, {u_theta, Nv, &src.u_theta}, {u_phi, N, &src.u_phi}};
+    for (int k = 0; k < 4 && rc == SB_OK; ++k)
+        if (in[k].from) {
+            rc = copy_f64(b, k, in[k].from, in[k].n);
+            *in[k].to = f64_buffer(b, k);
+        }
+    if (rc == SB_OK) rc = reset_bimocq(b, src);
     if (rc == SB_OK) {
         cudaError_t e = cudaStreamSynchronize(b->stream);
         if (e != cudaSuccess) rc = cuda_fail(e, "upload sync");
@@ -1185,11 +1206,10 @@ int sb_download_field_f32(sb_bubble* b, sb_field which, float* dst, size_t n) {
 int sb_synchronize(sb_bubble* b) {
     if (!b) return fail(SB_ERR_INVALID, "null handle");
     SB_CHECK(cudaSetDevice(b->device));
+    // with the outcome of the most recent solve (none before the first step)
+    SB_CHECK(cudaMemcpyAsync(b->h_stats, b->f.stats, sizeof(SbDevStats), cudaMemcpyDeviceToHost, b->stream));
     SB_CHECK(cudaStreamSynchronize(b->stream));
-    // the outcome of the most recent solve (none before the first step)
-    SbDevStats st;
-    SB_CHECK(cudaMemcpy(&st, b->f.stats, sizeof(st), cudaMemcpyDeviceToHost));
-    if (st.solves > 0 && !st.solver_converged)
+    if (b->h_stats->solves > 0 && !b->h_stats->solver_converged)
         return fail(SB_ERR_NOT_CONVERGED, "the last implicit solve missed its tolerance");
     return SB_OK;
 }
@@ -1447,6 +1467,8 @@ struct sb_batch {
     cudaStream_t stream = nullptr;
     char* arena = nullptr;
     SbStepPlan plan{};  // the members as one set: their own descriptors, tiles, solve set
+    SbStepParams* h_params = nullptr;  // every member's step scalars, pinned
+    SbStepParams* d_params = nullptr;  // and on the device
     cudaGraphExec_t graph = nullptr;
     cudaEvent_t ev[STAGE_COUNT + 1] = {};
     long long steps = 0;
@@ -1462,11 +1484,16 @@ int batch_set_params_each(sb_batch* B, const double* t, double dt) {
     for (size_t k = 0; k < B->m.size() && same; ++k)
         same = B->m[k]->last_t == t[k] && B->m[k]->last_dt == dt;
     if (same) return SB_OK;
-    SB_CHECK(cudaStreamSynchronize(B->stream));  // pinned slots may be in flight
+    SB_CHECK(cudaStreamSynchronize(B->stream));  // the pinned array may be in flight
     for (size_t k = 0; k < B->m.size(); ++k) {
-        int rc = write_step_params(B->m[k], t[k], dt, B->stream);
-        if (rc != SB_OK) return rc;
+        step_params(B->m[k], t[k], dt, B->h_params + k);
+        B->m[k]->last_dt = dt;
+        B->m[k]->last_t = t[k];
     }
+    // one copy and one kernel for all members
+    SB_CHECK(cudaMemcpyAsync(B->d_params, B->h_params, sizeof(SbStepParams) * B->m.size(),
+                             cudaMemcpyHostToDevice, B->stream));
+    SB_CHECK(launch_set_params(B->plan.descs, B->d_params, (int)B->m.size(), B->stream));
     return SB_OK;
 }
 
@@ -1569,8 +1596,10 @@ int sb_batch_create(sb_bubble* const* bubbles, int n, sb_batch** out) {
                  o_rec = L.take(sizeof(SbSolveRec) * 2 * n), o_done = L.take(sizeof(int) * n),
                  o_cnt = L.take(sizeof(int) * n),
                  o_acc = L.take(sizeof(unsigned long long) * kSolveAccWords * n),
-                 o_bar = L.take(sizeof(unsigned) * kGridBarWords);
+                 o_bar = L.take(sizeof(unsigned) * kGridBarWords),
+                 o_params = L.take(sizeof(SbStepParams) * n);
     e = cudaMalloc((void**)&B->arena, L.bytes);
+    if (e == cudaSuccess) e = cudaMallocHost((void**)&B->h_params, sizeof(SbStepParams) * n);
     if (e == cudaSuccess) e = cudaMemset(B->arena, 0, L.bytes);
     if (e != cudaSuccess) {
         int r = cuda_fail(e, "sb_batch_create allocation");
@@ -1600,6 +1629,7 @@ int sb_batch_create(sb_bubble* const* bubbles, int n, sb_batch** out) {
     S.cnt = (int*)(A + o_cnt);
     S.acc = (unsigned long long*)(A + o_acc);
     S.bar = (unsigned*)(A + o_bar);
+    B->d_params = (SbStepParams*)(A + o_params);
     // members may have work queued on their own streams; a member retired
     // from an earlier batch takes part again
     for (sb_bubble* b : B->m) e = e == cudaSuccess ? cudaStreamSynchronize(b->stream) : e;
@@ -1629,6 +1659,7 @@ int sb_batch_destroy(sb_batch* B) {
     for (cudaEvent_t e : B->ev)
         if (e) cudaEventDestroy(e);
     if (B->arena) cudaFree(B->arena);
+    if (B->h_params) cudaFreeHost(B->h_params);
     if (B->stream) cudaStreamDestroy(B->stream);
     delete B;
     return SB_OK;

@@ -133,12 +133,25 @@ enum SbStage {
     STAGE_COUNT
 };
 
-cudaError_t launch_reset_maps(const SbGrid& g, const SbFields& f, cudaStream_t s);
+// Uploaded FP64 arrays on the device; null: the field is kept.
+struct SbRestart {
+    const double *eta, *gamma, *u_theta, *u_phi;
+};
+// New fields, BIMOCQ buffers and maps restarted from them (and from the kept ones).
+cudaError_t launch_restart(const SbGrid& g, const SbFields& f, const SbRestart& src, const SbPhys& ph,
+                           int storage, cudaStream_t s);
+// params[k] into member k's step scalars (device arrays).
+cudaError_t launch_set_params(SbBubbleDesc* const* descs, const SbStepParams* params, int nb,
+                              cudaStream_t s);
 cudaError_t launch_mass(const SbGrid& g, const SbPhys& ph, const SbFields& f, int storage,
                         cudaStream_t s);
 // FP32 <-> stored thickness / surfactant field (n elements, offset `base`).
 cudaError_t launch_store(SbScalar* dst, const float* src, int n, float base, int storage,
                          cudaStream_t s);
+// An FP64 device array, or a constant, into a stored field (FP32 arrays: kStoreF32, base 0).
+cudaError_t launch_store_f64(SbScalar* dst, const double* src, int n, float base, int storage,
+                             cudaStream_t s);
+cudaError_t launch_fill(SbScalar* dst, float v, int n, float base, int storage, cudaStream_t s);
 cudaError_t launch_load(float* dst, const SbScalar* src, int n, float base, int storage,
                         cudaStream_t s);
 

@@ -1098,13 +1098,37 @@ __global__ void k_barrier_probe(SbBubbleDesc* d, int absent, unsigned limit) {
     grid_barrier(d->f.bar, gen, gridDim.x, &d->f.stats->wait_faults, limit);
 }
 
-__global__ void k_reset_maps(SbGrid g, SbFields f) {
+// A new state: the fields given (FP64, as uploaded) take their stored type,
+// the BIMOCQ buffers and the maps restart from thickness and surfactant, and
+// the next solve starts from dx = 0 (the state it would warm-start from has
+// been replaced).
+template <class T>
+__global__ void k_restart(SbGrid g, SbFields f, SbRestart src, float base_eta, float base_gam) {
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= g.N) return;
+    if (src.eta) st_s<T>(f.eta, idx, (float)src.eta[idx], base_eta);
+    if (src.gamma) st_s<T>(f.gam, idx, (float)src.gamma[idx], base_gam);
+    if (src.u_phi) f.uph[idx] = (float)src.u_phi[idx];
+    if (src.u_theta && idx < g.Nv) f.uth[idx] = (float)src.u_theta[idx];
+    cp_s<T>(f.eta_init, f.eta, idx);
+    cp_s<T>(f.eta_initL, f.eta, idx);
+    cp_s<T>(f.gam_init, f.gam, idx);
+    cp_s<T>(f.gam_initL, f.gam, idx);
+    f.eta_delta[idx] = 0.0f;
+    f.eta_deltaL[idx] = 0.0f;
+    f.gam_delta[idx] = 0.0f;
+    f.gam_deltaL[idx] = 0.0f;
     const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     f.fwd[0][idx] = z; f.fwd[1][idx] = z;
     f.bwd[0][idx] = z; f.bwd[1][idx] = z;
     f.bwdprev[idx] = z;
+    if (idx == 0) f.stats->dx_valid = 0;
+}
+
+// Step scalars of a batch's members to where their kernels read them.
+__global__ void k_set_params(SbBubbleDesc* const* descs, const SbStepParams* params, int nb) {
+    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b < nb) *descs[b]->f.step = params[b];
 }
 
 __device__ __forceinline__ double warp_sum_d(double v) {
@@ -1136,6 +1160,17 @@ template <class T>
 __global__ void k_store(SbScalar* __restrict__ dst, const float* __restrict__ src, int n, float base) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) st_s<T>(dst, i, src[i], base);
+}
+// An uploaded FP64 array, or a constant, in its stored type.
+template <class T>
+__global__ void k_store_f64(SbScalar* __restrict__ dst, const double* __restrict__ src, int n, float base) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) st_s<T>(dst, i, (float)src[i], base);
+}
+template <class T>
+__global__ void k_fill(SbScalar* dst, float v, int n, float base) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) st_s<T>(dst, i, v, base);
 }
 template <class T>
 __global__ void k_load(float* __restrict__ dst, const SbScalar* __restrict__ src, int n, float base) {
@@ -1252,8 +1287,17 @@ cudaError_t launch_plan_step(const SbStepPlan& P, cudaStream_t s) {
     return launch_plan_flip(P, s);
 }
 
-cudaError_t launch_reset_maps(const SbGrid& g, const SbFields& f, cudaStream_t s) {
-    k_reset_maps<<<(g.N + kBlock - 1) / kBlock, kBlock, 0, s>>>(g, f);
+cudaError_t launch_restart(const SbGrid& g, const SbFields& f, const SbRestart& src, const SbPhys& ph,
+                           int storage, cudaStream_t s) {
+    const int nb = (g.N + kBlock - 1) / kBlock;
+    if (storage == kStoreBF16) k_restart<__nv_bfloat16><<<nb, kBlock, 0, s>>>(g, f, src, ph.base_eta, ph.base_gam);
+    else k_restart<float><<<nb, kBlock, 0, s>>>(g, f, src, ph.base_eta, ph.base_gam);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_set_params(SbBubbleDesc* const* descs, const SbStepParams* params, int nb,
+                              cudaStream_t s) {
+    k_set_params<<<(nb + kBlock - 1) / kBlock, kBlock, 0, s>>>(descs, params, nb);
     return cudaGetLastError();
 }
 
@@ -1272,6 +1316,21 @@ cudaError_t launch_store(SbScalar* dst, const float* src, int n, float base, int
     const int nb = (n + kBlock - 1) / kBlock;
     if (storage == kStoreBF16) k_store<__nv_bfloat16><<<nb, kBlock, 0, s>>>(dst, src, n, base);
     else k_store<float><<<nb, kBlock, 0, s>>>(dst, src, n, base);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_store_f64(SbScalar* dst, const double* src, int n, float base, int storage,
+                             cudaStream_t s) {
+    const int nb = (n + kBlock - 1) / kBlock;
+    if (storage == kStoreBF16) k_store_f64<__nv_bfloat16><<<nb, kBlock, 0, s>>>(dst, src, n, base);
+    else k_store_f64<float><<<nb, kBlock, 0, s>>>(dst, src, n, base);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_fill(SbScalar* dst, float v, int n, float base, int storage, cudaStream_t s) {
+    const int nb = (n + kBlock - 1) / kBlock;
+    if (storage == kStoreBF16) k_fill<__nv_bfloat16><<<nb, kBlock, 0, s>>>(dst, v, n, base);
+    else k_fill<float><<<nb, kBlock, 0, s>>>(dst, v, n, base);
     return cudaGetLastError();
 }
 
