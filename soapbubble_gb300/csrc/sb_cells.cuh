@@ -107,6 +107,60 @@ __device__ __forceinline__ const SbBubbleDesc& stage_tile_desc(SbBubbleDesc* con
     return *s_d;
 }
 
+// The bubble of a block: its descriptor, its first cell, the map parity.  A
+// bubble stepped alone comes in the kernel's parameters (ONE: its pointers and
+// constants are then uniform operands, and nothing is staged: three dependent
+// loads and a barrier per block), the cells in block order; what changes on
+// the device is read there (the parity, the halt switch, and the offsets of
+// BF16 fields, which an upload moves).  A set's blocks find theirs by tile.
+struct StepBlock {
+    int first, cur;
+    bool halted;
+    float base_eta, base_gam;
+};
+template <bool ONE>
+__device__ __forceinline__ const SbBubbleDesc& step_block(const SbBubbleDesc& one,
+                                                          SbBubbleDesc* const* descs,
+                                                          const int2* tiles, int tile_cells,
+                                                          SbBubbleDesc* s_d, StepBlock& B) {
+    if (ONE) {
+        const SbBubbleDesc* self = one.f.self;
+        B.first = blockIdx.x * tile_cells;
+        B.cur = self->cur;
+        B.halted = self->halted != 0;
+        B.base_eta = self->ph.base_eta;
+        B.base_gam = self->ph.base_gam;
+        return one;
+    }
+    const int2 t = tiles[blockIdx.x];
+    const SbBubbleDesc& d = stage_tile_desc(descs, t.x, s_d);
+    B.first = t.y;
+    B.cur = d.cur;
+    B.halted = d.halted != 0;
+    B.base_eta = d.ph.base_eta;
+    B.base_gam = d.ph.base_gam;
+    return d;
+}
+
+#define SB_STEP_ARGS                                                                           \
+    const __grid_constant__ SbBubbleDesc one, SbBubbleDesc* const* __restrict__ descs,         \
+        const int2* __restrict__ tiles, int tile_cells
+#define SB_STEP_BLOCK(cells)                                                                   \
+    __shared__ __align__(16) SbBubbleDesc s_d[1];                                              \
+    StepBlock B;                                                                               \
+    const SbBubbleDesc& d = step_block<ONE>(one, descs, tiles, cells, s_d, B);                 \
+    if (B.halted) return; /* the same in every thread of the block */
+
+// One launch over `blocks` tiles of size `tile` from tile `first` on.
+template <class K>
+void launch_cells(const SbStepPlan& P, int first, int blocks, int tile, int threads, K* one, K* each,
+                  cudaStream_t s) {
+    static const SbBubbleDesc none{};  // a batch: the kernels find their bubble by tile
+    const int2* tiles = P.tiles[tile] + first;
+    if (P.one) one<<<blocks, threads, 0, s>>>(*P.one, P.descs, tiles, kTileSizes[tile]);
+    else each<<<blocks, threads, 0, s>>>(none, P.descs, tiles, kTileSizes[tile]);
+}
+
 }  // namespace
 
 }  // namespace sb

@@ -307,46 +307,12 @@ __device__ __forceinline__ bool round_trip_fast(const SbBubbleDesc& d, int cur, 
     return ok & (far <= kSlerpFar);
 }
 
-// The block's bubble: its descriptor (ONE: in kernel parameters, cells in
-// block order; else staged by tile), first cell and map parity.
-struct ChainBlock {
-    int first, cur;
-    bool halted;
-};
-template <bool ONE>
-__device__ __forceinline__ const SbBubbleDesc& chain_block(const SbBubbleDesc& one,
-                                                           SbBubbleDesc* const* descs,
-                                                           const int2* tiles, int tile_cells,
-                                                           SbBubbleDesc* s_d, ChainBlock& B) {
-    if (ONE) {
-        B.first = blockIdx.x * tile_cells;
-        B.cur = one.f.self->cur;
-        B.halted = one.f.self->halted != 0;
-        return one;
-    }
-    const int2 t = tiles[blockIdx.x];
-    const SbBubbleDesc& d = stage_tile_desc(descs, t.x, s_d);
-    B.first = t.y;
-    B.cur = d.cur;
-    B.halted = d.halted != 0;
-    return d;
-}
-
-#define SB_CHAIN_ARGS                                                                          \
-    const __grid_constant__ SbBubbleDesc one, SbBubbleDesc* const* __restrict__ descs,         \
-        const int2* __restrict__ tiles, int tile_cells
-#define SB_CHAIN_BLOCK                                                                         \
-    __shared__ __align__(16) SbBubbleDesc s_d[1];                                              \
-    ChainBlock B;                                                                              \
-    const SbBubbleDesc& d = chain_block<ONE>(one, descs, tiles, tile_cells, s_d, B);           \
-    if (B.halted) return;  /* the same in every thread of the block */                         \
-    const int cur = B.cur;
-
 // PAR = 1: a thread per cell runs the cell's chains side by side; PAR = 2: a
 // thread per cell and chain, chain by chain in whole warps.
 template <bool ONE, int PAR>
-__global__ void __launch_bounds__(256 * PAR, PAR == 1 ? 5 : 2) k_advect_maps_chains(SB_CHAIN_ARGS) {
-    SB_CHAIN_BLOCK
+__global__ void __launch_bounds__(256 * PAR, PAR == 1 ? 5 : 2) k_advect_maps_chains(SB_STEP_ARGS) {
+    SB_STEP_BLOCK(tile_cells)
+    const int cur = B.cur;
     const int chain = PAR == 1 ? -1 : threadIdx.x / tile_cells;
     const int idx = B.first + (int)threadIdx.x - (PAR == 1 ? 0 : chain * tile_cells);
     if (idx >= d.g.N) return;
@@ -368,8 +334,9 @@ __global__ void __launch_bounds__(256 * PAR, PAR == 1 ? 5 : 2) k_advect_maps_cha
     if (chain != 0 && maps && !ahead) forward_general(d, cur, idx);
 }
 template <bool ONE, int PAR>
-__global__ void __launch_bounds__(256 * PAR, PAR == 1 ? 5 : 2) k_velocity_chains(SB_CHAIN_ARGS) {
-    SB_CHAIN_BLOCK
+__global__ void __launch_bounds__(256 * PAR, PAR == 1 ? 5 : 2) k_velocity_chains(SB_STEP_ARGS) {
+    SB_STEP_BLOCK(tile_cells)
+    const int cur = B.cur;
     (void)cur;
     const int chain = PAR == 1 ? -1 : threadIdx.x / tile_cells;
     const int idx = B.first + (int)threadIdx.x - (PAR == 1 ? 0 : chain * tile_cells);
@@ -389,9 +356,10 @@ constexpr int kSampleCells = 64;  // cells of a block with its samples in parall
 // PAR = 1: the tile's cells, one per thread; PAR = 5: a pair of warps per
 // sample point; the first pair adds the samples up in their order.
 template <bool ONE, int PAR>
-__global__ void __launch_bounds__(PAR == 1 ? 256 : 5 * kSampleCells, 4) k_bimocq_chains(SB_CHAIN_ARGS) {
+__global__ void __launch_bounds__(PAR == 1 ? 256 : 5 * kSampleCells, 4) k_bimocq_chains(SB_STEP_ARGS) {
     __shared__ float2 s_t[5][PAR == 1 ? 1 : kSampleCells];
-    SB_CHAIN_BLOCK
+    SB_STEP_BLOCK(tile_cells)
+    const int cur = B.cur;
     if (d.ph.plain_adv) return;  // thickness advected by k_advect_maps
     const SbGrid& g = d.g;
     const float blend = d.ph.blend;
@@ -494,12 +462,13 @@ __device__ __forceinline__ void accum_store(const SbFields& f, int idx, const Ac
 }
 
 template <bool ONE, int PAR>
-__global__ void __launch_bounds__(PAR == 1 ? 256 : 6 * kSampleCells, 4) k_accum_chains(SB_CHAIN_ARGS) {
+__global__ void __launch_bounds__(PAR == 1 ? 256 : 6 * kSampleCells, 4) k_accum_chains(SB_STEP_ARGS) {
     __shared__ float4 s_v[5][PAR == 1 ? 1 : kSampleCells];
     __shared__ unsigned s_far;
     if (threadIdx.x == 0) s_far = 0u;
     if (ONE) __syncthreads();
-    SB_CHAIN_BLOCK
+    SB_STEP_BLOCK(tile_cells)
+    const int cur = B.cur;
     const SbGrid& g = d.g;
     const SbFields& f = d.f;
     const float2 th = __ldg(&g.rottab[g.nT + 1]);
@@ -589,16 +558,10 @@ namespace {
 // (512 x 1024: k_bimocq 49 us against 58, k_accum 39 against 53).
 constexpr int kChipThreads = 152 * 1024;
 
-// Grid, block and cells per block of one launch: PAR chains of a cell in
-// parallel, or the set's tiles of size tile.
+// PAR chains of a cell in parallel over the set's tiles of size tile.
 template <class K>
 void launch_chains(const SbStepPlan& P, int tile, int par, K* one, K* each, cudaStream_t s) {
-    static const SbBubbleDesc none{};  // a batch: the kernels find their bubble by tile
-    const int cells = kTileSizes[tile], blocks = P.nchain[tile];
-    if (P.one)
-        one<<<blocks, cells * par, 0, s>>>(*P.one, P.descs, P.tiles[tile], cells);
-    else
-        each<<<blocks, cells * par, 0, s>>>(none, P.descs, P.tiles[tile], cells);
+    launch_cells(P, 0, P.nchain[tile], tile, kTileSizes[tile] * par, one, each, s);
 }
 
 }  // namespace

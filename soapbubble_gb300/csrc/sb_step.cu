@@ -35,9 +35,8 @@ constexpr int kBlock = 128;
 
 // ---------------------------------------------------------------------------
 template <class T>
-__device__ __forceinline__ void advect_maps_cell(const SbGrid& g, const SbPhys& ph, const SbFields& f, int cur,
-                                          int idx) {
-    (void)cur;
+__device__ __forceinline__ void advect_maps_cell(const SbGrid& g, const SbPhys& ph, const StepBlock& B,
+                                                 const SbFields& f, int cur, int idx) {
     const int i = idx >> g.logP, j = idx & g.maskP;
     const float dt = f.step->dt;
     const Frame F = cell_frame(g, i, j);
@@ -50,8 +49,8 @@ __device__ __forceinline__ void advect_maps_cell(const SbGrid& g, const SbPhys& 
         // backward trace; the maps are not used
         const Trace Tb = trace_gc(g, f.uth, f.uph, F, gt, gp, dt);
         const SStencil sb = sstencil_of(g, centred_stencil(g, pos_of(F, Tb, g), 0.0f));
-        f.eta_adv[idx] = gather_s<T>(f.eta, sb, ph.base_eta);
-        f.gam_adv[idx] = gather_s<T>(f.gam, sb, ph.base_gam);
+        f.eta_adv[idx] = gather_s<T>(f.eta, sb, B.base_eta);
+        f.gam_adv[idx] = gather_s<T>(f.gam, sb, B.base_gam);
     } else {
         // forward map: trace forward in time (negative step), sample the old map
         const Trace Tf = trace_gc(g, f.uth, f.uph, F, gt, gp, -dt);
@@ -63,15 +62,13 @@ __device__ __forceinline__ void advect_maps_cell(const SbGrid& g, const SbPhys& 
         const CStencil cb = centred_stencil(g, pos_of(F, Tb, g), 0.0f);
         const f3 db = map_at_stencil(g, f.bwd[cur], F, cb);
         f.bwd[cur ^ 1][idx] = make_float4(db.x, db.y, db.z, 0.0f);
-        f.gam_adv[idx] = gather_s<T>(f.gam, sstencil_of(g, cb), ph.base_gam);
+        f.gam_adv[idx] = gather_s<T>(f.gam, sstencil_of(g, cb), B.base_gam);
     }
 
     step_start(g, f, idx);
 }
 
-__device__ __forceinline__ void velocity_cell(const SbGrid& g, const SbPhys& ph, const SbFields& f, int cur,
-                                          int idx) {
-    (void)cur;
+__device__ __forceinline__ void velocity_cell(const SbGrid& g, const SbPhys& ph, const SbFields& f, int idx) {
     f.uph_adv[idx] = velocity_uphi(g, ph, f, idx);
     if ((idx >> g.logP) < g.nT - 1) f.uth_adv[idx] = velocity_utheta(g, ph, f, idx);
 }
@@ -79,12 +76,11 @@ __device__ __forceinline__ void velocity_cell(const SbGrid& g, const SbPhys& ph,
 // BIMOCQ thickness: compose the new backward map with the previous one and
 // blend the two reconstructions (MULTISAMPLE, 5 samples).
 template <class T>
-__device__ __forceinline__ void bimocq_cell(const SbGrid& g, const SbPhys& ph, const SbFields& f, int cur,
-                                          int idx) {
-    (void)cur;
+__device__ __forceinline__ void bimocq_cell(const SbGrid& g, const SbPhys& ph, const StepBlock& B,
+                                            const SbFields& f, int cur, int idx) {
     if (ph.plain_adv) return;  // thickness advected by k_advect_maps
     const int i = idx >> g.logP, j = idx & g.maskP;
-    const float be = ph.base_eta;
+    const float be = B.base_eta;
     if (ld_s<T>(f.eta, idx, be) == 0.0f) {
         f.eta_adv[idx] = 0.0f;
         return;
@@ -429,9 +425,7 @@ __device__ __forceinline__ void assemble_broken(const SbFields& f, float gmax, i
 }
 
 template <bool VISC>
-__device__ __forceinline__ void assemble_cell(const SbGrid& g, const SbPhys& ph, const SbFields& f, int cur,
-                                          int idx) {
-    (void)cur;
+__device__ __forceinline__ void assemble_cell(const SbGrid& g, const SbPhys& ph, const SbFields& f, int idx) {
     const int i = idx >> g.logP, j = idx & g.maskP;
     const int nP = g.nP, nT = g.nT;
     const float mixA = f.step->mixA, mixB = f.step->mixB;
@@ -618,9 +612,8 @@ __device__ __forceinline__ float gnew_diff(const SbFields& f, int a, int b, floa
 }
 
 template <class T, bool VISC>
-__device__ __forceinline__ void post_cell(const SbGrid& g, const SbPhys& ph, const SbFields& f, int cur,
-                                          int idx) {
-    (void)cur;
+__device__ __forceinline__ void post_cell(const SbGrid& g, const SbPhys& ph, const StepBlock& B,
+                                          const SbFields& f, int idx) {
     const int i = idx >> g.logP, j = idx & g.maskP;
     const int nP = g.nP;
     const float dt = f.step->dt, invDt = f.step->invDt;
@@ -629,12 +622,12 @@ __device__ __forceinline__ void post_cell(const SbGrid& g, const SbPhys& ph, con
     const float gNew = f.x[idx];
     float mdtdiv;  // -dt * div
     if (gamma_clamped(gNew, ph.gthr)) {
-        st_s<T>(f.gam, idx, gmax, ph.base_gam);
+        st_s<T>(f.gam, idx, gmax, B.base_gam);
         f.d_gam[idx] = gmax - gOld;
         mdtdiv = -1.0f;
     } else {
         const float dx = f.dx[idx];
-        st_s<T>(f.gam, idx, gNew, ph.base_gam);
+        st_s<T>(f.gam, idx, gNew, B.base_gam);
         f.d_gam[idx] = dx;
         // div = (1 - min(gNew, 2 gOld) / gOld) / dt
         mdtdiv = (gNew > 2.0f * gOld) ? 1.0f : dx / gOld;
@@ -643,10 +636,10 @@ __device__ __forceinline__ void post_cell(const SbGrid& g, const SbPhys& ph, con
     const float e = f.eta_adv[idx];
     const float de = e * mdtdiv + f.step->evapDt;
     if (e + de >= 0.0f) {
-        st_s<T>(f.eta, idx, e + de, ph.base_eta);
+        st_s<T>(f.eta, idx, e + de, B.base_eta);
         f.d_eta[idx] = de;
     } else {
-        st_s<T>(f.eta, idx, 0.0f, ph.base_eta);
+        st_s<T>(f.eta, idx, 0.0f, B.base_eta);
         f.d_eta[idx] = -e;
     }
 
@@ -717,8 +710,8 @@ __device__ __forceinline__ float gnew_diff_v(float xa, float2 da, float ga, floa
 // (the west neighbour of the first cell in scalar ones), and each cell
 // does post_cell's operations.
 template <class T>
-__device__ __forceinline__ void post_quad(const SbGrid& g, const SbPhys& ph, const SbFields& f,
-                                          int idx, int chains) {
+__device__ __forceinline__ void post_quad(const SbGrid& g, const SbPhys& ph, const StepBlock& B,
+                                          const SbFields& f, int idx, int chains) {
     const int i = idx >> g.logP, j = idx & g.maskP;
     const int nP = g.nP;
     const float invDt = f.step->invDt, evapDt = f.step->evapDt;
@@ -793,8 +786,8 @@ __device__ __forceinline__ void post_quad(const SbGrid& g, const SbPhys& ph, con
             }
         }
     }
-    st4_s<T>(f.gam, idx, oG, ph.base_gam);
-    st4_s<T>(f.eta, idx, oE, ph.base_eta);
+    st4_s<T>(f.gam, idx, oG, B.base_gam);
+    st4_s<T>(f.eta, idx, oE, B.base_eta);
     if (chains) {
 #pragma unroll
         for (int k = 0; k < 4; ++k)
@@ -814,8 +807,8 @@ __device__ __forceinline__ void post_quad(const SbGrid& g, const SbPhys& ph, con
 // re-initialisation, when the distortion calls for it, only corrects.
 // returns the cell's distortion (0 outside the grid)
 template <class T>
-__device__ __forceinline__ float accum_cell(const SbGrid& g, const SbPhys& ph, const SbFields& f, int cur,
-                                           int idx) {
+__device__ __forceinline__ float accum_cell(const SbGrid& g, const StepBlock& B, const SbFields& f, int cur,
+                                            int idx) {
     const int i = idx >> g.logP, j = idx & g.maskP;
     const Frame F = cell_frame(g, i, j);
     const float4* fwd = f.fwd[cur ^ 1];
@@ -832,13 +825,13 @@ __device__ __forceinline__ float accum_cell(const SbGrid& g, const SbPhys& ph, c
         const SStencil s = sstencil_of(g, c);
         ed += kW5[k] * gather(f.d_eta, s);
         gd += kW5[k] * gather(f.d_gam, s);
-        th += kW5[k] * gather_s<T>(f.eta, s, ph.base_eta);
-        gm += kW5[k] * gather_s<T>(f.gam, s, ph.base_gam);
+        th += kW5[k] * gather_s<T>(f.eta, s, B.base_eta);
+        gm += kW5[k] * gather_s<T>(f.gam, s, B.base_gam);
     }
     f.eta_delta[idx] = ed;
     f.gam_delta[idx] = gd;
-    f.err_eta[idx] = (th - ed - ld_s<T>(f.eta_init, idx, ph.base_eta)) * 0.5f;
-    f.err_gam[idx] = (gm - gd - ld_s<T>(f.gam_init, idx, ph.base_gam)) * 0.5f;
+    f.err_eta[idx] = (th - ed - ld_s<T>(f.eta_init, idx, B.base_eta)) * 0.5f;
+    f.err_gam[idx] = (gm - gd - ld_s<T>(f.gam_init, idx, B.base_gam)) * 0.5f;
     // estimateDistortion: dist(x, bwd(fwd(x))) and dist(x, fwd(bwd(x))); fwd(x)
     // is sample 4 above (the cell's own map entry), whose stencil is reused
     const float d1 = dist_from_disp(map_at_stencil(g, bwd, F, c4), g.invh);
@@ -872,91 +865,76 @@ __device__ __forceinline__ void block_max_distortion(float dist, SbDevStats* st)
 // Kernels whose cells touch the stored thickness / surfactant fields are
 // instantiated per storage type T (float or __nv_bfloat16); a plan launches
 // the instantiation of its bubbles' storage.
-#define SB_CELL_KERNEL_BODY(...)                                                       \
-    __shared__ __align__(16) SbBubbleDesc s_d;                                         \
-    const int2 t = tiles[blockIdx.x];                                                  \
-    const SbBubbleDesc& d = stage_tile_desc(descs, t.x, &s_d);                         \
-    if (d.halted) return;                                                              \
-    const int idx = t.y + threadIdx.x;                                                 \
-    if (idx < d.g.N) __VA_ARGS__(d.g, d.ph, d.f, d.cur, idx);
-
-#define SB_CELL_KERNEL(name)                                                           \
-    __global__ void __launch_bounds__(256) k_##name(SbBubbleDesc* const* __restrict__ descs, \
-                                                    const int2* __restrict__ tiles) {  \
-        SB_CELL_KERNEL_BODY(name##_cell)                                               \
-    }
-
 // k_advect_maps is held to 48 registers per thread (five 256-thread blocks
 // per SM; a few spilled values): measured 61 -> 58 us on c1.
-template <class T>
-__global__ void __launch_bounds__(256, 5) k_advect_maps(SbBubbleDesc* const* __restrict__ descs,
-                                                        const int2* __restrict__ tiles) {
-    SB_CELL_KERNEL_BODY(advect_maps_cell<T>)
+template <class T, bool ONE>
+__global__ void __launch_bounds__(256, 5) k_advect_maps(SB_STEP_ARGS) {
+    SB_STEP_BLOCK(tile_cells)
+    const int idx = B.first + threadIdx.x;
+    if (idx < d.g.N) advect_maps_cell<T>(d.g, d.ph, B, d.f, B.cur, idx);
 }
-SB_CELL_KERNEL(velocity)
+template <bool ONE>
+__global__ void __launch_bounds__(256) k_velocity(SB_STEP_ARGS) {
+    SB_STEP_BLOCK(tile_cells)
+    const int idx = B.first + threadIdx.x;
+    if (idx < d.g.N) velocity_cell(d.g, d.ph, d.f, idx);
+}
 // k_bimocq is held to 64 registers per thread with its five samples taken two
 // at a time (two independent map-lookup chains in flight per thread; a few
 // spilled values): measured 79.7 -> 75.9 us on c1 (either change alone, or
 // all five samples unrolled, is slower).
-template <class T>
-__global__ void __launch_bounds__(256, 4) k_bimocq(SbBubbleDesc* const* __restrict__ descs,
-                                                   const int2* __restrict__ tiles) {
-    SB_CELL_KERNEL_BODY(bimocq_cell<T>)
+template <class T, bool ONE>
+__global__ void __launch_bounds__(256, 4) k_bimocq(SB_STEP_ARGS) {
+    SB_STEP_BLOCK(tile_cells)
+    const int idx = B.first + threadIdx.x;
+    if (idx < d.g.N) bimocq_cell<T>(d.g, d.ph, B, d.f, B.cur, idx);
 }
 // k_assemble / k_post: the instantiations with VISC = true evaluate the
 // viscous forces (every bubble of a plan has the same switch).
-template <bool VISC>
-__global__ void __launch_bounds__(256) k_assemble(SbBubbleDesc* const* __restrict__ descs,
-                                                  const int2* __restrict__ tiles) {
-    SB_CELL_KERNEL_BODY(assemble_cell<VISC>)
+template <bool VISC, bool ONE>
+__global__ void __launch_bounds__(256) k_assemble(SB_STEP_ARGS) {
+    SB_STEP_BLOCK(tile_cells)
+    const int idx = B.first + threadIdx.x;
+    if (idx < d.g.N) assemble_cell<VISC>(d.g, d.ph, d.f, idx);
 }
 
 // The non-viscous assembly, four cells per thread (a tile of n cells runs
 // in n / 4 threads), held to 64 registers: c1 16.4 us as one cell per
 // thread, c2 49.2 us against 51.2 (uncapped, 114 registers: 18.4 and 49.0).
-__global__ void __launch_bounds__(64, 16) k_assemble4(SbBubbleDesc* const* __restrict__ descs,
-                                                  const int2* __restrict__ tiles) {
-    __shared__ __align__(16) SbBubbleDesc s_d;
-    const int2 t = tiles[blockIdx.x];
-    const SbBubbleDesc& d = stage_tile_desc(descs, t.x, &s_d);
-    if (d.halted) return;
-    const int idx = t.y + 4 * threadIdx.x;
+template <bool ONE>
+__global__ void __launch_bounds__(64, 16) k_assemble4(SB_STEP_ARGS) {
+    SB_STEP_BLOCK(tile_cells)
+    const int idx = B.first + 4 * threadIdx.x;
     if (idx < d.g.N) assemble_quad(d.g, d.ph, d.f, idx);
 }
 
-template <class T, bool VISC>
-__global__ void __launch_bounds__(256) k_post(SbBubbleDesc* const* __restrict__ descs,
-                                              const int2* __restrict__ tiles) {
-    SB_CELL_KERNEL_BODY(post_cell<T, VISC>)
-    if (d.chains && idx < d.g.N)  // what the accumulation's chains sample, in one word
+template <class T, bool VISC, bool ONE>
+__global__ void __launch_bounds__(256) k_post(SB_STEP_ARGS) {
+    SB_STEP_BLOCK(tile_cells)
+    const int idx = B.first + threadIdx.x;
+    if (idx >= d.g.N) return;
+    post_cell<T, VISC>(d.g, d.ph, B, d.f, idx);
+    if (d.chains)  // what the accumulation's chains sample, in one word
         d.f.changes[idx] = make_float4(d.f.d_eta[idx], d.f.d_gam[idx], ld_s<T>(d.f.eta, idx, 0.0f),
                                        ld_s<T>(d.f.gam, idx, 0.0f));
 }
 
 // The non-viscous post-solve update, four cells per thread (a tile of n
 // cells runs in n / 4 threads).
-template <class T>
-__global__ void __launch_bounds__(64) k_post4(SbBubbleDesc* const* __restrict__ descs,
-                                              const int2* __restrict__ tiles) {
-    __shared__ __align__(16) SbBubbleDesc s_d;
-    const int2 t = tiles[blockIdx.x];
-    const SbBubbleDesc& d = stage_tile_desc(descs, t.x, &s_d);
-    if (d.halted) return;
-    const int idx = t.y + 4 * threadIdx.x;
-    if (idx < d.g.N) post_quad<T>(d.g, d.ph, d.f, idx, d.chains);
+template <class T, bool ONE>
+__global__ void __launch_bounds__(64) k_post4(SB_STEP_ARGS) {
+    SB_STEP_BLOCK(tile_cells)
+    const int idx = B.first + 4 * threadIdx.x;
+    if (idx < d.g.N) post_quad<T>(d.g, d.ph, B, d.f, idx, d.chains);
 }
 
 // k_accum is held to 64 registers per thread (a few spilled values): the
 // occupancy it gains outweighs them (measured 87 -> 84 us on c1).
-template <class T>
-__global__ void __launch_bounds__(256, 4) k_accum(SbBubbleDesc* const* __restrict__ descs,
-                                               const int2* __restrict__ tiles) {
-    __shared__ __align__(16) SbBubbleDesc s_d;
-    const int2 t = tiles[blockIdx.x];
-    const SbBubbleDesc& d = stage_tile_desc(descs, t.x, &s_d);
-    if (d.halted) return;  // the same in every thread of the block
-    const int idx = t.y + threadIdx.x;
-    const float dist = idx < d.g.N ? accum_cell<T>(d.g, d.ph, d.f, d.cur, idx) : 0.0f;
+template <class T, bool ONE>
+__global__ void __launch_bounds__(256, 4) k_accum(SB_STEP_ARGS) {
+    SB_STEP_BLOCK(tile_cells)
+    const int idx = B.first + threadIdx.x;
+    const float dist = idx < d.g.N ? accum_cell<T>(d.g, B, d.f, B.cur, idx) : 0.0f;
     block_max_distortion(dist, d.f.stats);
 }
 
@@ -1208,47 +1186,44 @@ cudaError_t prepare_plan(const SbStepPlan& P) {
 cudaError_t launch_plan_stage(const SbStepPlan& P, int stage, cudaStream_t s) {
     const int k = P.sel[stage];
     const int n = P.ntiles[k], block = kTileSizes[k];
-    SbBubbleDesc* const* d = P.descs;
-    const int2* t = P.tiles[k];
     const bool bf = P.storage == kStoreBF16;
     // the tiles of the members the chain kernels serve come first
     const int nc = P.nchain[k], nr = n - nc;
-    const int2* tr = t + nc;
+    // a launch over the tiles from `from` on, `per` cells per thread
+#define SB_LAUNCH(from, count, per, one, each) launch_cells(P, from, count, k, block / (per), one, each, s)
+    using bf16 = __nv_bfloat16;
     switch (stage) {
         case STAGE_MAPS:
             if (nc) launch_chain_stage(P, stage, s);
-            if (nr && bf) k_advect_maps<__nv_bfloat16><<<nr, block, 0, s>>>(d, tr);
-            else if (nr) k_advect_maps<float><<<nr, block, 0, s>>>(d, tr);
+            if (nr && bf) SB_LAUNCH(nc, nr, 1, (k_advect_maps<bf16, true>), (k_advect_maps<bf16, false>));
+            else if (nr) SB_LAUNCH(nc, nr, 1, (k_advect_maps<float, true>), (k_advect_maps<float, false>));
             break;
         case STAGE_VELOCITY:
             if (nc) launch_chain_stage(P, stage, s);
-            if (nr) k_velocity<<<nr, block, 0, s>>>(d, tr);
+            if (nr) SB_LAUNCH(nc, nr, 1, k_velocity<true>, k_velocity<false>);
             break;
         case STAGE_BIMOCQ:
             if (nc) launch_chain_stage(P, stage, s);
-            if (nr && bf) k_bimocq<__nv_bfloat16><<<nr, block, 0, s>>>(d, tr);
-            else if (nr) k_bimocq<float><<<nr, block, 0, s>>>(d, tr);
+            if (nr && bf) SB_LAUNCH(nc, nr, 1, (k_bimocq<bf16, true>), (k_bimocq<bf16, false>));
+            else if (nr) SB_LAUNCH(nc, nr, 1, (k_bimocq<float, true>), (k_bimocq<float, false>));
             break;
         case STAGE_ASSEMBLE:
-            if (P.viscous) k_assemble<true><<<n, block, 0, s>>>(d, t);
-            else k_assemble4<<<n, block / 4, 0, s>>>(d, t);
+            if (P.viscous) SB_LAUNCH(0, n, 1, (k_assemble<true, true>), (k_assemble<true, false>));
+            else SB_LAUNCH(0, n, 4, k_assemble4<true>, k_assemble4<false>);
             break;
         case STAGE_SOLVE:
             return P.one ? launch_solve_one(P.one->g, P.one->f, P.set, P.solver, s)
                          : launch_solve(P.set, P.maxNP, P.solver, s);
         case STAGE_POST:
-            if (P.viscous) {
-                if (bf) k_post<__nv_bfloat16, true><<<n, block, 0, s>>>(d, t);
-                else k_post<float, true><<<n, block, 0, s>>>(d, t);
-            } else {
-                if (bf) k_post4<__nv_bfloat16><<<n, block / 4, 0, s>>>(d, t);
-                else k_post4<float><<<n, block / 4, 0, s>>>(d, t);
-            }
+            if (P.viscous && bf) SB_LAUNCH(0, n, 1, (k_post<bf16, true, true>), (k_post<bf16, true, false>));
+            else if (P.viscous) SB_LAUNCH(0, n, 1, (k_post<float, true, true>), (k_post<float, true, false>));
+            else if (bf) SB_LAUNCH(0, n, 4, (k_post4<bf16, true>), (k_post4<bf16, false>));
+            else SB_LAUNCH(0, n, 4, (k_post4<float, true>), (k_post4<float, false>));
             break;
         case STAGE_ACCUM:
             if (nc) launch_chain_stage(P, stage, s);
-            if (nr && bf) k_accum<__nv_bfloat16><<<nr, block, 0, s>>>(d, tr);
-            else if (nr) k_accum<float><<<nr, block, 0, s>>>(d, tr);
+            if (nr && bf) SB_LAUNCH(nc, nr, 1, (k_accum<bf16, true>), (k_accum<bf16, false>));
+            else if (nr) SB_LAUNCH(nc, nr, 1, (k_accum<float, true>), (k_accum<float, false>));
             break;
         case STAGE_REINIT: {
             // the re-initialisation works on kBlock-cell tiles
