@@ -264,7 +264,8 @@ __device__ __forceinline__ float bound_off(float v, float lim) {
     return fmaxf(fminf(v, lim), -lim);
 }
 
-__device__ __forceinline__ CStencil centred_stencil(const SbGrid& g, Pos q, float colOff) {
+// Positions that may lie across a pole or are not finite.
+static __device__ __noinline__ CStencil centred_stencil_any(const SbGrid& g, Pos q, float colOff) {
     CStencil s;
     int bi = q.bi, bj = q.bj;
     float ox = bound_off(q.ox, 4.0f * g.nT);
@@ -298,6 +299,26 @@ __device__ __forceinline__ CStencil centred_stencil(const SbGrid& g, Pos q, floa
         s.r1 = hi; s.v1 = false; s.c10 = j0; s.c11 = j1;
     }
     return s;
+}
+
+// The stencil of a position between two rows of the grid in a few steps (no
+// unfolding, no reflected row: the same values as the general form, which
+// serves the others).
+__device__ __forceinline__ CStencil centred_stencil(const SbGrid& g, Pos q, float colOff) {
+    const float t = q.ox - 0.5f, kf = floorf(t);
+    const int lo = q.bi + (int)kf;
+    if ((unsigned)lo < (unsigned)(g.nT - 1) && fabsf(q.ox) <= 4.0f * g.nT && fabsf(q.oy) <= 4.0f * g.nP) {
+        CStencil s;
+        const float ty = q.oy - colOff, kj = floorf(ty);
+        const int j0 = (q.bj + (int)kj) & g.maskP, j1 = (j0 + 1) & g.maskP;
+        s.r0 = lo; s.r1 = lo + 1;
+        s.c00 = s.c10 = j0; s.c01 = s.c11 = j1;
+        s.v0 = s.v1 = s.flipped = false;
+        s.a = t - kf;
+        s.b = ty - kj;
+        return s;
+    }
+    return centred_stencil_any(g, q, colOff);
 }
 
 // Scalar or u_phi sample (sampleCentered kernel/bubble.cu:320-376, sampleVPhi
