@@ -13,6 +13,7 @@
 // gamma's rounding over h sin(theta)), of which another rounding of gamma
 // changes a tenth.
 
+#define SB_SHORT_FORMS 0
 #include "sb_cells.cuh"
 #include "sb_fastgeo.cuh"
 #include "sb_internal.h"

@@ -42,6 +42,19 @@
 #ifndef SB_CONV_INLINE
 #define SB_CONV_INLINE __noinline__
 #endif
+// Stencils and velocity samples have a short form for positions between two
+// rows and call the general one for the others.  The chain kernels, which come
+// here only for their special cases, take the general forms inline
+// (SB_SHORT_FORMS 0: with calls below their own call k_advect_maps_chains
+// took 37.4 us in place of 34.9 at 512 x 1024).
+#ifndef SB_SHORT_FORMS
+#define SB_SHORT_FORMS 1
+#endif
+#if SB_SHORT_FORMS
+#define SB_ANY_INLINE __noinline__
+#else
+#define SB_ANY_INLINE __forceinline__
+#endif
 
 namespace sb {
 
@@ -265,7 +278,7 @@ __device__ __forceinline__ float bound_off(float v, float lim) {
 }
 
 // Positions that may lie across a pole or are not finite.
-static __device__ __noinline__ CStencil centred_stencil_any(const SbGrid& g, Pos q, float colOff) {
+static __device__ SB_ANY_INLINE CStencil centred_stencil_any(const SbGrid& g, Pos q, float colOff) {
     CStencil s;
     int bi = q.bi, bj = q.bj;
     float ox = bound_off(q.ox, 4.0f * g.nT);
@@ -305,6 +318,7 @@ static __device__ __noinline__ CStencil centred_stencil_any(const SbGrid& g, Pos
 // unfolding, no reflected row: the same values as the general form, which
 // serves the others).
 __device__ __forceinline__ CStencil centred_stencil(const SbGrid& g, Pos q, float colOff) {
+#if SB_SHORT_FORMS
     const float t = q.ox - 0.5f, kf = floorf(t);
     const int lo = q.bi + (int)kf;
     if ((unsigned)lo < (unsigned)(g.nT - 1) && fabsf(q.ox) <= 4.0f * g.nT && fabsf(q.oy) <= 4.0f * g.nP) {
@@ -318,15 +332,16 @@ __device__ __forceinline__ CStencil centred_stencil(const SbGrid& g, Pos q, floa
         s.b = ty - kj;
         return s;
     }
+#endif
     return centred_stencil_any(g, q, colOff);
 }
 
 // Scalar or u_phi sample (sampleCentered kernel/bubble.cu:320-376, sampleVPhi
 // 178-240).  VEC: across-pole rows and flipped positions change sign.
 template <bool VEC>
-__device__ __forceinline__ float sample_centred(const SbGrid& g, const float* __restrict__ f,
-                                                Pos q, float colOff) {
-    const CStencil s = centred_stencil(g, q, colOff);
+static __device__ SB_ANY_INLINE float sample_centred_any(const SbGrid& g, const float* __restrict__ f,
+                                                        Pos q, float colOff) {
+    const CStencil s = centred_stencil_any(g, q, colOff);
     const int nP = g.nP;
     const float f00 = f[s.r0 * nP + s.c00], f01 = f[s.r0 * nP + s.c01];
     const float f10 = f[s.r1 * nP + s.c10], f11 = f[s.r1 * nP + s.c11];
@@ -350,6 +365,21 @@ __device__ __forceinline__ float sample_centred(const SbGrid& g, const float* __
     return r;
 }
 
+template <bool VEC>
+__device__ __forceinline__ float sample_centred(const SbGrid& g, const float* __restrict__ f,
+                                                Pos q, float colOff) {
+#if SB_SHORT_FORMS
+    const float t = q.ox - 0.5f, kf = floorf(t);
+    const int lo = q.bi + (int)kf;
+    if ((unsigned)lo < (unsigned)(g.nT - 1) && fabsf(q.ox) <= 4.0f * g.nT && fabsf(q.oy) <= 4.0f * g.nP) {
+        const float a = t - kf, ty = q.oy - colOff, kj = floorf(ty), b = ty - kj;
+        const int j0 = (q.bj + (int)kj) & g.maskP, j1 = (j0 + 1) & g.maskP, nP = g.nP;
+        return bilerp(f[lo * nP + j0], f[lo * nP + j1], f[(lo + 1) * nP + j0], f[(lo + 1) * nP + j1], a, b);
+    }
+#endif
+    return sample_centred_any<VEC>(g, f, q, colOff);
+}
+
 __device__ __forceinline__ float sample_scalar(const SbGrid& g, const float* __restrict__ f, Pos q) {
     return sample_centred<false>(g, f, q, 0.0f);
 }
@@ -360,7 +390,7 @@ __device__ __forceinline__ float sample_uphi(const SbGrid& g, const float* __res
 // u_theta sample (sampleVTheta, kernel/bubble.cu:247-313).  Rows sit at raw
 // theta i + 1, i = 0..nT-2; next to a pole the nearest samples are the row and
 // its across-pole reflection two cells away.
-__device__ __forceinline__ float sample_utheta(const SbGrid& g, const float* __restrict__ f, Pos q) {
+static __device__ SB_ANY_INLINE float sample_utheta_any(const SbGrid& g, const float* __restrict__ f, Pos q) {
     int bi = q.bi, bj = q.bj;
     float ox = bound_off(q.ox, 4.0f * g.nT);
     q.oy = bound_off(q.oy, 4.0f * g.nP);
@@ -395,6 +425,20 @@ __device__ __forceinline__ float sample_utheta(const SbGrid& g, const float* __r
                    a, b);
     }
     return flipped ? -r : r;
+}
+
+// Between two rows of faces: the last case in a few steps.
+__device__ __forceinline__ float sample_utheta(const SbGrid& g, const float* __restrict__ f, Pos q) {
+#if SB_SHORT_FORMS
+    const float kf = floorf(q.ox);
+    const int lo = q.bi - 1 + (int)kf;
+    if ((unsigned)lo < (unsigned)(g.nT - 2) && fabsf(q.ox) <= 4.0f * g.nT && fabsf(q.oy) <= 4.0f * g.nP) {
+        const float a = q.ox - kf, kj = floorf(q.oy), b = q.oy - kj;
+        const int j0 = (q.bj + (int)kj) & g.maskP, j1 = (j0 + 1) & g.maskP, nP = g.nP;
+        return bilerp(f[lo * nP + j0], f[lo * nP + j1], f[(lo + 1) * nP + j0], f[(lo + 1) * nP + j1], a, b);
+    }
+#endif
+    return sample_utheta_any(g, f, q);
 }
 
 // Displacement, in the cell frame F, of the map point stored for cell
