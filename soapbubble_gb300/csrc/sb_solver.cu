@@ -1110,16 +1110,38 @@ __device__ __forceinline__ void advance(const SbSolveSet& S, int b, int p, const
     S.cnt[b] = 0;
 }
 
-// Work weight of one theta row of a system with nT rows (nP = 2 nT columns
-// plus a fixed per-row cost of about 256 columns).
-__device__ __forceinline__ unsigned row_weight(int nT) { return 2u * (unsigned)nT + 256u; }
+// Cost of one theta row of nP columns in a phase of kind `kind`, in units of
+// 64 cycles as measured on sets of 17 and 35 members (a block's share of its
+// SM): a set-up row takes four to five times a q = A p row, and systems that
+// iterate side by side are at different kinds.  Equal weights for all kinds
+// left the blocks waiting at the barrier for 40 % of the solve.
+__device__ __forceinline__ unsigned row_weight(int kind, int nP) {
+    unsigned fixed = 60, per64 = 8;  // K_Q
+    switch (kind) {
+        case K_SETUP: fixed = 110; per64 = 31; break;
+        case K_SETUP_L: fixed = 110; per64 = 37; break;
+        case K_NEUMANN: fixed = 95; per64 = 10; break;
+        case K_UPDATE: case K_RESTART: fixed = 80; per64 = 8; break;
+        case K_UPDATE_L: case K_RESTART_L: fixed = 86; per64 = 7; break;
+        case K_CHECK: per64 = 12; break;
+        default: break;
+    }
+    return fixed + per64 * (unsigned)nP / 64u;
+}
 
-// s_pre[b] = total weight of the systems before b that are active in phase
-// p (every system in phase 0 and in the final pass, p < 0); s_pre[nb] is the
-// total.  Every block computes the same table: a system's done_at only
-// moves during phase p from INT_MAX to p + 1, which reads as active in p.
+// A system's part in a phase, as every block of the set sees it.
+struct SetShared {
+    unsigned pre[kMaxSystems + 1];     // weight of the systems before, the total last
+    unsigned short rows[kMaxSystems];  // rows; 0: retired from its batch (halted), takes no part
+    unsigned char kind[kMaxSystems];   // kind in the phase
+};
+
+// H.pre: weights of the systems active in phase p (every system in phase 0 and
+// in the final pass, p < 0).  Every block computes the same table: a system's
+// done_at only moves during phase p from INT_MAX to p + 1, which reads as
+// active in p, and its record of phase p is written in phase p - 1.
 template <int TB>
-__device__ __forceinline__ unsigned active_prefix(const SbSolveSet& S, int p, unsigned* s_pre) {
+__device__ __forceinline__ unsigned active_prefix(const SbSolveSet& S, int p, SetShared& H) {
     __shared__ unsigned wsum[TB / 32];
     __shared__ unsigned carry;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -1129,9 +1151,14 @@ __device__ __forceinline__ unsigned active_prefix(const SbSolveSet& S, int p, un
         const int b = base + threadIdx.x;
         unsigned v = 0;
         if (b < S.nb) {
-            // a member retired from its batch (halted) takes no part
-            const bool act = (p <= 0 || __ldcg(&S.done_at[b]) > p) && !__ldcg(&S.descs[b]->halted);
-            if (act) v = (unsigned)(S.roff[b + 1] - S.roff[b]) * row_weight(S.roff[b + 1] - S.roff[b]);
+            int kind = p < 0 ? K_Q : H.kind[b];
+            bool act = true;
+            if (p > 0) {
+                act = __ldcg(&S.done_at[b]) > p;
+                kind = __ldcg(&S.rec[(p & 1) * S.nb + b].kind);
+                H.kind[b] = (unsigned char)kind;
+            }
+            if (act) v = H.rows[b] * row_weight(kind, 2 * H.rows[b]);
         }
         unsigned incl = v;
 #pragma unroll
@@ -1143,13 +1170,13 @@ __device__ __forceinline__ unsigned active_prefix(const SbSolveSet& S, int p, un
         __syncthreads();
         unsigned before = carry;
         for (int k = 0; k < w; ++k) before += wsum[k];
-        if (b < S.nb) s_pre[b] = before + incl - v;
+        if (b < S.nb) H.pre[b] = before + incl - v;
         __syncthreads();
         if (threadIdx.x == TB - 1) carry = before + incl;
         __syncthreads();
     }
     const unsigned total = carry;
-    if (threadIdx.x == 0) s_pre[S.nb] = total;
+    if (threadIdx.x == 0) H.pre[S.nb] = total;
     __syncthreads();
     return total;
 }
@@ -1324,7 +1351,7 @@ __device__ __forceinline__ void row_phase(const SbGrid& g, const SbFields& f,
 // record (set-up, then per iteration q = A p, update, Neumann term; in
 // mixed mode the refinement check and restart).  In
 // every phase the rows of the systems still iterating are split into G
-// contiguous ranges of equal work weight, one per block, so a block meets
+// contiguous ranges of equal cost (row_weight), one per block, so a block meets
 // one or two systems per phase and a system that iterates longer than the
 // others still spreads over the whole GPU.  Each block adds its rows'
 // partials into the system's exact accumulator and counts the rows; the
@@ -1336,7 +1363,7 @@ k_solve(SbSolveSet S, SolverConfig cfg) {
     extern __shared__ __align__(16) float sm[];
     __shared__ __align__(8) uint64_t bar;
     __shared__ __align__(16) SbBubbleDesc s_d;
-    __shared__ unsigned s_pre[kMaxSystems + 1];
+    __shared__ SetShared H;
     __shared__ int s_last;
     __shared__ unsigned long long s_w[3 * kAccWords];
     __shared__ ff s_sums[3];
@@ -1348,17 +1375,23 @@ k_solve(SbSolveSet S, SolverConfig cfg) {
     Stage St;
     stage_init(St, &bar, sm, cfg.blob);
     const unsigned G = gridDim.x;
+    const unsigned* const s_pre = H.pre;
+    for (int b = threadIdx.x; b < S.nb; b += TB) {
+        const SbBubbleDesc* d = S.descs[b];
+        H.rows[b] = d->halted ? 0 : (unsigned short)(S.roff[b + 1] - S.roff[b]);
+        H.kind[b] = (unsigned char)first_kind(d->f.stats, cfg);
+    }
 
     for (int p = 0;; ++p) {
-        const unsigned W = active_prefix<TB>(S, p, s_pre);
+        const unsigned W = active_prefix<TB>(S, p, H);
         if (W == 0) break;  // same in every block
         const unsigned lo = (unsigned)(((unsigned long long)W * blockIdx.x) / G);
         const unsigned hi = (unsigned)(((unsigned long long)W * (blockIdx.x + 1)) / G);
         for (int b = first_system_after(s_pre, S.nb, lo); b < S.nb && s_pre[b] < hi; ++b) {
             const unsigned w0 = s_pre[b];
             if (s_pre[b + 1] == w0) continue;  // not active
-            const int nT = S.roff[b + 1] - S.roff[b];
-            const unsigned wr = row_weight(nT);
+            const int nT = H.rows[b];
+            const unsigned wr = (s_pre[b + 1] - w0) / (unsigned)nT;
             // rows whose start weight w0 + i wr lies in [lo, hi)
             const int i0 = lo > w0 ? (int)((lo - w0 + wr - 1) / wr) : 0;
             const int i1 = min(nT, (int)((hi - w0 + wr - 1) / wr));
@@ -1367,13 +1400,12 @@ k_solve(SbSolveSet S, SolverConfig cfg) {
             // grid reads the same record), staged with the descriptor
             if (threadIdx.x == 0) {
                 SbSolveRec rc;
-                rc.kind = p == 0 ? first_kind(S.descs[b]->f.stats, cfg) : K_SETUP;
+                rc.kind = H.kind[b];
                 rc.it = 0;
                 rc.beta = 0.0f;
                 rc.alpha = make_float2(0.0f, 0.0f);
                 if (p > 0) {
                     const SbSolveRec* rp = S.rec + (p & 1) * S.nb + b;
-                    rc.kind = __ldcg(&rp->kind);
                     rc.it = __ldcg(&rp->it);
                     rc.beta = __ldcg(&rp->beta);
                     rc.alpha = __ldcg(&rp->alpha);
@@ -1416,13 +1448,14 @@ k_solve(SbSolveSet S, SolverConfig cfg) {
     }
     // the increment and the new gamma of every system, same split with all
     // systems counted
-    const unsigned W = active_prefix<TB>(S, -1, s_pre);
+    const unsigned W = active_prefix<TB>(S, -1, H);
     const unsigned lo = (unsigned)(((unsigned long long)W * blockIdx.x) / G);
     const unsigned hi = (unsigned)(((unsigned long long)W * (blockIdx.x + 1)) / G);
     for (int b = first_system_after(s_pre, S.nb, lo); b < S.nb && s_pre[b] < hi; ++b) {
         const unsigned w0 = s_pre[b];
-        const int nT = S.roff[b + 1] - S.roff[b];
-        const unsigned wr = row_weight(nT);
+        if (s_pre[b + 1] == w0) continue;  // retired
+        const int nT = H.rows[b];
+        const unsigned wr = (s_pre[b + 1] - w0) / (unsigned)nT;
         const int i0 = lo > w0 ? (int)((lo - w0 + wr - 1) / wr) : 0;
         const int i1 = min(nT, (int)((hi - w0 + wr - 1) / wr));
         if (i0 >= i1) continue;
