@@ -314,7 +314,7 @@ template <bool ONE, int PAR>
 __global__ void __launch_bounds__(256 * PAR, PAR == 1 ? 5 : 2) k_advect_maps_chains(SB_STEP_ARGS) {
     SB_STEP_BLOCK(tile_cells)
     const int cur = B.cur;
-    const int chain = PAR == 1 ? -1 : threadIdx.x / tile_cells;
+    const int chain = PAR == 1 ? -1 : (int)threadIdx.x / tile_cells;
     const int idx = B.first + (int)threadIdx.x - (PAR == 1 ? 0 : chain * tile_cells);
     if (idx >= d.g.N) return;
     const bool inner = inner_row(d.g, idx >> d.g.logP), maps = !d.ph.plain_adv;
@@ -339,7 +339,7 @@ __global__ void __launch_bounds__(256 * PAR, PAR == 1 ? 5 : 2) k_velocity_chains
     SB_STEP_BLOCK(tile_cells)
     const int cur = B.cur;
     (void)cur;
-    const int chain = PAR == 1 ? -1 : threadIdx.x / tile_cells;
+    const int chain = PAR == 1 ? -1 : (int)threadIdx.x / tile_cells;
     const int idx = B.first + (int)threadIdx.x - (PAR == 1 ? 0 : chain * tile_cells);
     if (idx >= d.g.N) return;
     const int i = idx >> d.g.logP;

@@ -232,7 +232,8 @@ cudaError_t launch_plan_stage(const SbStepPlan& P, int stage, cudaStream_t s);
 // chain kernels serve (sb_chain.cu).
 void launch_chain_stage(const SbStepPlan& P, int stage, cudaStream_t s);
 cudaError_t launch_plan_flip(const SbStepPlan& P, cudaStream_t s);
-cudaError_t launch_plan_step(const SbStepPlan& P, cudaStream_t s);
+cudaError_t launch_plan_step(const SbStepPlan& P, cudaStream_t s, cudaStream_t side, cudaEvent_t fork,
+                             cudaEvent_t join);
 // Self-test of the bounded grid barrier on a bubble's barrier word (`blocks`
 // co-resident blocks, block `absent` never arrives; sb_step.cu).
 cudaError_t launch_barrier_probe(SbBubbleDesc* d, int blocks, int absent, unsigned limit,

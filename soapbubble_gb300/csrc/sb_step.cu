@@ -1254,12 +1254,19 @@ cudaError_t launch_plan_flip(const SbStepPlan& P, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_plan_step(const SbStepPlan& P, cudaStream_t s) {
-    for (int st = 0; st < STAGE_COUNT; ++st) {
-        cudaError_t e = launch_plan_stage(P, st, s);
-        if (e != cudaSuccess) return e;
-    }
-    return launch_plan_flip(P, s);
+cudaError_t launch_plan_step(const SbStepPlan& P, cudaStream_t s, cudaStream_t side, cudaEvent_t fork,
+                             cudaEvent_t join) {
+    // the velocities need nothing of the map and thickness stages: a branch of
+    // the captured step beside them, until the assembly
+    cudaError_t e = cudaEventRecord(fork, s);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(side, fork, 0);
+    if (e == cudaSuccess) e = launch_plan_stage(P, STAGE_MAPS, s);
+    if (e == cudaSuccess) e = launch_plan_stage(P, STAGE_VELOCITY, side);
+    if (e == cudaSuccess) e = cudaEventRecord(join, side);
+    if (e == cudaSuccess) e = launch_plan_stage(P, STAGE_BIMOCQ, s);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(s, join, 0);
+    for (int st = STAGE_ASSEMBLE; st < STAGE_COUNT && e == cudaSuccess; ++st) e = launch_plan_stage(P, st, s);
+    return e == cudaSuccess ? launch_plan_flip(P, s) : e;
 }
 
 cudaError_t launch_restart(const SbGrid& g, const SbFields& f, const SbRestart& src, const SbPhys& ph,
