@@ -652,6 +652,16 @@ template <>
 __device__ __forceinline__ void st_s<__nv_bfloat16>(SbScalar* p, int i, float v, float base) {
     reinterpret_cast<__nv_bfloat16*>(p)[i] = __float2bfloat16_rn(v - base);
 }
+// What a load returns of a value v stored.
+template <class T>
+__device__ __forceinline__ float as_stored(float v, float base) {
+    (void)base;
+    return v;
+}
+template <>
+__device__ __forceinline__ float as_stored<__nv_bfloat16>(float v, float base) {
+    return base + __bfloat162float(__float2bfloat16_rn(v - base));
+}
 // Element copy between two fields of the same base (exact).
 template <class T>
 __device__ __forceinline__ void cp_s(SbScalar* dst, const SbScalar* src, int i) {

@@ -59,15 +59,16 @@ struct SbFields {
     float4 *fwd[2], *bwd[2], *bwdprev;
     float *uair_init, *vair_init, *corr_u, *corr_v;
     float *uair, *vair;                            // N+1, Nv+1 (last element 0)
-    float *d_eta, *d_gam, *err_eta, *err_gam;  // per-step increments, re-initialisation errors
+    float *d_eta, *d_gam;                          // the re-initialisation's corrected fields
+    float *err_eta, *err_gam;                      // and their errors
     // implicit system for the increment dx = gamma_new - gamma_adv:
     // (A dx)_c = dmass_c dx_c + sum_n w_cn (dx_c - dx_n), weights w > 0 to
     // the east (cE) and south (cS) neighbours; r = b - A gamma_adv formed
     // analytically; rhs = b (for the norm only)
     float *dmass, *cE, *cS, *rhs, *r0;
     float *x, *dx, *r, *z, *z1, *p, *q;            // solver vectors
-    // sampled together by the chain kernels; they lie over z, z1, p
-    // and q, which are dead outside the solve
+    // sampled together (eta_near and eta_far by the chain kernels); they lie
+    // over z, z1, p and q, which are dead outside the solve
     float2* eta_near;                              // (init, delta) of the thickness (z, z1)
     float* eta_far;                                // initL + deltaL of the thickness (p)
     float4* changes;                               // (d_eta, d_gam, eta, gam) after the solve (z .. q)

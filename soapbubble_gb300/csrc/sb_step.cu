@@ -90,7 +90,8 @@ __device__ __forceinline__ void bimocq_cell(const SbGrid& g, const SbPhys& ph, c
     f3 d1s[5];
     sample_map_multi5(g, f.bwd[cur ^ 1], F, d1s);
     float attrib = 0.0f;
-#pragma unroll 2
+    constexpr int kUnroll = sizeof(T) == 4 ? 2 : 1;  // see k_bimocq
+#pragma unroll kUnroll
     for (int k = 0; k < 5; ++k) {
         const CStencil c1 = centred_stencil(g, pos_from_disp_fast(F, d1s[k], g.invh, g.nT), 0.0f);
         const f3 d2 = map_at_stencil(g, f.bwdprev, F, c1);
@@ -589,6 +590,7 @@ __device__ __forceinline__ void assemble_quad(const SbGrid& g, const SbPhys& ph,
 // update, thickness update with evaporation, and the per-step changes that
 // BIMOCQ accumulates.  Increments are carried directly (dx from the solve,
 // d_eta = -eta dt div + evap dt) instead of as differences of O(1) values.
+// changes holds what the accumulation samples, the fields as they were stored.
 // Neighbouring new gamma values are clamped on the fly exactly as
 // divergenceKernel_fromGamma clamps them in place (kernel/bubble.cu:1287;
 // thr as in is_broken).
@@ -621,14 +623,15 @@ __device__ __forceinline__ void post_cell(const SbGrid& g, const SbPhys& ph, con
     const float gOld = f.gam_adv[idx];
     const float gNew = f.x[idx];
     float mdtdiv;  // -dt * div
+    float4 ch;
     if (gamma_clamped(gNew, ph.gthr)) {
-        st_s<T>(f.gam, idx, gmax, B.base_gam);
-        f.d_gam[idx] = gmax - gOld;
+        ch.w = gmax;
+        ch.y = gmax - gOld;
         mdtdiv = -1.0f;
     } else {
         const float dx = f.dx[idx];
-        st_s<T>(f.gam, idx, gNew, B.base_gam);
-        f.d_gam[idx] = dx;
+        ch.w = gNew;
+        ch.y = dx;
         // div = (1 - min(gNew, 2 gOld) / gOld) / dt
         mdtdiv = (gNew > 2.0f * gOld) ? 1.0f : dx / gOld;
     }
@@ -636,12 +639,17 @@ __device__ __forceinline__ void post_cell(const SbGrid& g, const SbPhys& ph, con
     const float e = f.eta_adv[idx];
     const float de = e * mdtdiv + f.step->evapDt;
     if (e + de >= 0.0f) {
-        st_s<T>(f.eta, idx, e + de, B.base_eta);
-        f.d_eta[idx] = de;
+        ch.z = e + de;
+        ch.x = de;
     } else {
-        st_s<T>(f.eta, idx, 0.0f, B.base_eta);
-        f.d_eta[idx] = -e;
+        ch.z = 0.0f;
+        ch.x = -e;
     }
+    st_s<T>(f.gam, idx, ch.w, B.base_gam);
+    st_s<T>(f.eta, idx, ch.z, B.base_eta);
+    ch.z = as_stored<T>(ch.z, B.base_eta);
+    ch.w = as_stored<T>(ch.w, B.base_gam);
+    f.changes[idx] = ch;
 
     // u_phi face between (i, j-1) and (i, j).  Under VISCOUS the reference
     // launches its u_phi update with the u_theta layout (nTheta - 1 rows,
@@ -711,7 +719,7 @@ __device__ __forceinline__ float gnew_diff_v(float xa, float2 da, float ga, floa
 // does post_cell's operations.
 template <class T>
 __device__ __forceinline__ void post_quad(const SbGrid& g, const SbPhys& ph, const StepBlock& B,
-                                          const SbFields& f, int idx, int chains) {
+                                          const SbFields& f, int idx) {
     const int i = idx >> g.logP, j = idx & g.maskP;
     const int nP = g.nP;
     const float invDt = f.step->invDt, evapDt = f.step->evapDt;
@@ -788,14 +796,10 @@ __device__ __forceinline__ void post_quad(const SbGrid& g, const SbPhys& ph, con
     }
     st4_s<T>(f.gam, idx, oG, B.base_gam);
     st4_s<T>(f.eta, idx, oE, B.base_eta);
-    if (chains) {
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-            f.changes[idx + k] = make_float4(oDE[k], oDG[k], oE[k], oG[k]);
-    } else {
-        st4(f.d_gam + idx, oDG);
-        st4(f.d_eta + idx, oDE);
-    }
+    for (int k = 0; k < 4; ++k)
+        f.changes[idx + k] = make_float4(oDE[k], oDG[k], as_stored<T>(oE[k], B.base_eta),
+                                         as_stored<T>(oG[k], B.base_gam));
     st4(f.uph + idx, oU);
     if (hasS) st4(f.uth + idx, oV);
 }
@@ -823,10 +827,13 @@ __device__ __forceinline__ float accum_cell(const SbGrid& g, const StepBlock& B,
         const CStencil c = centred_stencil(g, pos_from_disp_fast(F, ds[k], g.invh, g.nT), 0.0f);
         if (k == 4) c4 = c;
         const SStencil s = sstencil_of(g, c);
-        ed += kW5[k] * gather(f.d_eta, s);
-        gd += kW5[k] * gather(f.d_gam, s);
-        th += kW5[k] * gather_s<T>(f.eta, s, B.base_eta);
-        gm += kW5[k] * gather_s<T>(f.gam, s, B.base_gam);
+        // d_eta, d_gam, eta, gam
+        const float4 v00 = f.changes[s.i00], v01 = f.changes[s.i01];
+        const float4 v10 = f.changes[s.i10], v11 = f.changes[s.i11];
+        ed += kW5[k] * bilerp(v00.x, v01.x, v10.x, v11.x, s.a, s.b);
+        gd += kW5[k] * bilerp(v00.y, v01.y, v10.y, v11.y, s.a, s.b);
+        th += kW5[k] * bilerp(v00.z, v01.z, v10.z, v11.z, s.a, s.b);
+        gm += kW5[k] * bilerp(v00.w, v01.w, v10.w, v11.w, s.a, s.b);
     }
     f.eta_delta[idx] = ed;
     f.gam_delta[idx] = gd;
@@ -881,8 +888,9 @@ __global__ void __launch_bounds__(256) k_velocity(SB_STEP_ARGS) {
 }
 // k_bimocq is held to 64 registers per thread with its five samples taken two
 // at a time (two independent map-lookup chains in flight per thread; a few
-// spilled values): measured 79.7 -> 75.9 us on c1 (either change alone, or
-// all five samples unrolled, is slower).
+// spilled values): 244 us at 1024 x 2048 against 248 one at a time.  With
+// BF16 fields, whose samples also decode their values, it spills more and one
+// at a time is the faster: 244 against 255.
 template <class T, bool ONE>
 __global__ void __launch_bounds__(256, 4) k_bimocq(SB_STEP_ARGS) {
     SB_STEP_BLOCK(tile_cells)
@@ -912,11 +920,7 @@ template <class T, bool VISC, bool ONE>
 __global__ void __launch_bounds__(256) k_post(SB_STEP_ARGS) {
     SB_STEP_BLOCK(tile_cells)
     const int idx = B.first + threadIdx.x;
-    if (idx >= d.g.N) return;
-    post_cell<T, VISC>(d.g, d.ph, B, d.f, idx);
-    if (d.chains)  // what the accumulation's chains sample, in one word
-        d.f.changes[idx] = make_float4(d.f.d_eta[idx], d.f.d_gam[idx], ld_s<T>(d.f.eta, idx, 0.0f),
-                                       ld_s<T>(d.f.gam, idx, 0.0f));
+    if (idx < d.g.N) post_cell<T, VISC>(d.g, d.ph, B, d.f, idx);
 }
 
 // The non-viscous post-solve update, four cells per thread (a tile of n
@@ -925,11 +929,14 @@ template <class T, bool ONE>
 __global__ void __launch_bounds__(64) k_post4(SB_STEP_ARGS) {
     SB_STEP_BLOCK(tile_cells)
     const int idx = B.first + 4 * threadIdx.x;
-    if (idx < d.g.N) post_quad<T>(d.g, d.ph, B, d.f, idx, d.chains);
+    if (idx < d.g.N) post_quad<T>(d.g, d.ph, B, d.f, idx);
 }
 
 // k_accum is held to 64 registers per thread (a few spilled values): the
-// occupancy it gains outweighs them (measured 87 -> 84 us on c1).
+// occupancy it gains outweighs them.  What a sample takes from the post-solve
+// fields is one word per corner (SbFields::changes): four loads and their
+// addresses instead of sixteen, and no decoding of BF16 values, 188 -> 173 us
+// at 1024 x 2048 (BF16 191 -> 171) for 5 more in k_post, which writes the word.
 template <class T, bool ONE>
 __global__ void __launch_bounds__(256, 4) k_accum(SB_STEP_ARGS) {
     SB_STEP_BLOCK(tile_cells)
