@@ -99,7 +99,7 @@ struct SbBubbleDesc {
     int chains;        // 1: the chain kernels serve this bubble (uses_chains)
 };
 
-// Whether the chain kernels (sb_step.cu) serve a bubble.
+// Whether the chain kernels (sb_chain.cu, which gives the reasons) serve a bubble.
 inline bool uses_chains(const SbGrid& g, int storage) {
     return storage == kStoreF32 && g.nT <= 512;
 }

@@ -867,13 +867,15 @@ __device__ __forceinline__ void block_max_distortion(float dist, SbDevStats* st)
 // Kernels.  A launch covers a set of bubbles (one bubble, or every bubble of
 // a batch): descs[k] points to bubble k's descriptor, and block b works on
 // the cells tiles[b] = (bubble, first cell) .. + blockDim.x - 1 (a tile never
-// straddles two bubbles).  One bubble stepped alone and inside a batch runs
-// the same kernels on the same descriptor.
+// straddles two bubbles).  A bubble stepped alone passes its descriptor as a
+// kernel parameter (ONE); both instantiations run the same cell functions, and
+// a bubble alone and inside a batch gives the same bits.
 // Kernels whose cells touch the stored thickness / surfactant fields are
 // instantiated per storage type T (float or __nv_bfloat16); a plan launches
 // the instantiation of its bubbles' storage.
 // k_advect_maps is held to 48 registers per thread (five 256-thread blocks
-// per SM; a few spilled values): measured 61 -> 58 us on c1.
+// per SM; a few spilled values): 130 us at 1024 x 2048, 136 with four blocks,
+// 128 with six.
 template <class T, bool ONE>
 __global__ void __launch_bounds__(256, 5) k_advect_maps(SB_STEP_ARGS) {
     SB_STEP_BLOCK(tile_cells)
@@ -908,7 +910,8 @@ __global__ void __launch_bounds__(256) k_assemble(SB_STEP_ARGS) {
 
 // The non-viscous assembly, four cells per thread (a tile of n cells runs
 // in n / 4 threads), held to 64 registers: c1 16.4 us as one cell per
-// thread, c2 49.2 us against 51.2 (uncapped, 114 registers: 18.4 and 49.0).
+// thread, c2 49.2 us against 51.2 (uncapped, 114 registers: 18.4 and 49.0);
+// 41.0 at c2 since a bubble alone has its descriptor in parameters.
 template <bool ONE>
 __global__ void __launch_bounds__(64, 16) k_assemble4(SB_STEP_ARGS) {
     SB_STEP_BLOCK(tile_cells)
