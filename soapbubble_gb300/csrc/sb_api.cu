@@ -234,12 +234,14 @@ ArenaPlan plan_arena(const SbGrid& g, int storage) {
     a.uair_init = a.L.take(N * F); a.vair_init = a.L.take(Nv * F);
     a.corr_u = a.L.take(N * F); a.corr_v = a.L.take(Nv * F);
     a.uair = a.L.take((N + 1) * F); a.vair = a.L.take((Nv + 1) * F);
-    a.d_eta = a.L.take(N * F); a.d_gam = a.L.take(N * F);
-    a.err_eta = a.L.take(N * F); a.err_gam = a.L.take(N * F);
+    // two arrays of one block: a landing place of N doubles (f64_buffer)
+    a.d_eta = a.L.take(2 * N * F); a.d_gam = a.d_eta + N * F;
+    a.err_eta = a.L.take(2 * N * F); a.err_gam = a.err_eta + N * F;
     a.dmass = a.L.take(N * F); a.cE = a.L.take(N * F); a.cS = a.L.take(N * F);
     a.rhs = a.L.take(N * F); a.r0 = a.L.take(N * F); a.x = a.L.take(N * F); a.dx = a.L.take(N * F);
     a.r = a.L.take(N * F);
-    a.z = a.L.take(N * F); a.z1 = a.L.take(N * F); a.p = a.L.take(N * F); a.q = a.L.take(N * F);
+    // one block: SbFields::changes lies over all four, eta_near over z and z1
+    a.z = a.L.take(4 * N * F); a.z1 = a.z + N * F; a.p = a.z1 + N * F; a.q = a.p + N * F;
     a.xff = a.L.take(N * 8);
     a.pcr = a.L.take((size_t)g.nT * factor_blob(g.nP).bytes);
     a.pcr_levels = a.L.take((size_t)g.nT * 4);
@@ -376,10 +378,9 @@ bool state_field(sb_field w) {
     return !(w == SB_UAIR_INIT || w == SB_VAIR_INIT || w == SB_UAIR || w == SB_VAIR);
 }
 
-// Device buffers for uploaded FP64 arrays (8 bytes a cell): the per-step
+// Landing places of uploaded FP64 arrays, N doubles each: the per-step
 // increments and errors and the solver's vectors, which only live inside a
-// step, while uploads run between steps on the bubble's stream.  The arrays
-// of a pair follow one another in the arena without a gap.
+// step, while uploads run between steps on the bubble's stream.
 double* f64_buffer(sb_bubble* b, int k) {
     float* const at[4] = {b->f.d_eta, b->f.err_eta, b->f.z, b->f.p};
     return (double*)at[k];
@@ -389,6 +390,7 @@ double* f64_buffer(sb_bubble* b, int k) {
 // them took 0.25 ms of a 512 x 1024 field's 0.3, a page-locked or pageable
 // copy of the doubles takes 0.035 and the kernel 0.01.
 int copy_f64(sb_bubble* b, int k, const double* src, size_t n) {
+    if (n > (size_t)b->g.N) return fail(SB_ERR_INVALID, "upload larger than its landing place");
     SB_CHECK(cudaMemcpyAsync(f64_buffer(b, k), src, n * sizeof(double), cudaMemcpyHostToDevice, b->stream));
     return SB_OK;
 }
@@ -401,11 +403,16 @@ int reset_bimocq(sb_bubble* b, const SbRestart& src = {}) {
 }
 
 int upload_f32(sb_bubble* b, float* dst, const double* src, size_t n) {
-    int rc = copy_f64(b, 0, src, n);
-    if (rc != SB_OK) return rc;
-    SB_CHECK(launch_store_f64(reinterpret_cast<SbScalar*>(dst), f64_buffer(b, 0), (int)n, 0.0f, kStoreF32,
-                              b->stream));
-    b->launches += 1;
+    // the air flow's arrays have one element more than a landing place may hold
+    const size_t room = (size_t)b->g.N;
+    for (size_t at = 0; at < n; at += room) {
+        const size_t m = std::min(room, n - at);
+        int rc = copy_f64(b, 0, src + at, m);
+        if (rc != SB_OK) return rc;
+        SB_CHECK(launch_store_f64(reinterpret_cast<SbScalar*>(dst + at), f64_buffer(b, 0), (int)m, 0.0f,
+                                  kStoreF32, b->stream));
+        b->launches += 1;
+    }
     SB_CHECK(cudaStreamSynchronize(b->stream));
     return SB_OK;
 }
@@ -583,8 +590,6 @@ int sb_create(const sb_params* p, sb_bubble** out) {
     f.dmass = F32(a.dmass); f.cE = F32(a.cE); f.cS = F32(a.cS); f.rhs = F32(a.rhs); f.r0 = F32(a.r0);
     f.x = F32(a.x); f.dx = F32(a.dx); f.r = F32(a.r); f.z = F32(a.z); f.z1 = F32(a.z1);
     f.p = F32(a.p); f.q = F32(a.q);
-    // z, z1, p, q follow one another without gaps: N * 4 bytes is a multiple
-    // of the 256 that the arena rounds to (N = 2 nTheta^2, nTheta >= 8)
     f.eta_near = (float2*)f.z; f.eta_far = f.p; f.changes = (float4*)f.z;
     f.xff = (float2*)(A + a.xff);
     f.pcr = (float*)(A + a.pcr);

@@ -1,0 +1,100 @@
+"""The library's host code on a CUDA runtime without a GPU (fake_cudart.cpp):
+what it copies and where to, what it launches, and what it does when a call
+fails.  Kernels do not run, so no values are checked here."""
+import ctypes as C
+import importlib.util
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CUDA_INC = "/usr/local/cuda/include"
+
+
+class Fake:
+    """The library linked with the fake runtime, and the runtime's log."""
+
+    def __init__(self, path):
+        from soapbubble_gb300 import _lib
+        spec = importlib.util.spec_from_file_location("fake_sb_lib", _lib.__file__)
+        self.m = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(self.m)
+        self.m.LIB_PATH = path
+        L = self.L = self.m.lib()
+        L.fake_log.restype = L.fake_graph_node.restype = C.c_char_p
+        L.fake_fail.argtypes = [C.c_char_p, C.c_int]
+
+    def log(self, kind=""):
+        lines = [self.L.fake_log(i).decode() for i in range(self.L.fake_log_size())]
+        return [l for l in lines if l.startswith(kind)]
+
+    def copies(self):
+        return [tuple(int(v) for v in l.split()[1:]) for l in self.log("copy")]  # (to, from, bytes)
+
+    def clear(self):
+        self.L.fake_clear()
+
+    def fail(self, name, nth=1):
+        self.L.fake_fail(name.encode(), nth)
+
+    def params(self, nT, **kw):
+        p = self.m.SbParams()
+        self.L.sb_default_params(C.byref(p))
+        p.nTheta = nT
+        for k, v in kw.items():
+            setattr(p, k, v)
+        return p
+
+    def bubble(self, nT, **kw):
+        h = C.c_void_p()
+        p = self.params(nT, **kw)
+        assert self.L.sb_create(C.byref(p), C.byref(h)) == 0, self.L.sb_last_error()
+        return h
+
+    def batch(self, members):
+        arr = (C.c_void_p * len(members))(*[m.value for m in members])
+        h = C.c_void_p()
+        assert self.L.sb_batch_create(arr, len(members), C.byref(h)) == 0, self.L.sb_last_error()
+        return h
+
+    def field(self, name):
+        return self.m.FIELD_ID[name]
+
+
+def dp(a):
+    return a.ctypes.data_as(C.POINTER(C.c_double))
+
+
+@pytest.fixture(scope="module")
+def fake(gpulib, tmp_path_factory):
+    from soapbubble_gb300 import build
+    objs = [os.path.join(build.BUILD, os.path.splitext(s)[0] + ".o") for s in build.LIB_SOURCES]
+    out = str(tmp_path_factory.mktemp("fake") / "libsb_fake.so")
+    subprocess.run(["g++", "-shared", "-fPIC", "-O1", "-std=c++17", "-Wl,-Bsymbolic", "-I", CUDA_INC,
+                    os.path.join(HERE, "fake_cudart.cpp"), *objs, "-o", out], check=True)
+    return Fake(out)
+
+
+@pytest.mark.parametrize("nT", [8, 64, 512])
+@pytest.mark.parametrize("name", ["uair", "vair", "u_phi", "eta"])
+def test_uploads_stay_inside_their_landing_place(fake, nT, name):
+    """An FP64 array lands in scratch between steps: no copy may reach the
+    landing place of another one (the four arrays of sb_upload_fields mark
+    where each begins)."""
+    h = fake.bubble(nT)
+    N = 2 * nT * nT
+    a = np.zeros(N + 1)
+    fake.clear()
+    assert fake.L.sb_upload_fields(h, dp(a), dp(a), dp(a), dp(a), None, None) == 0
+    places = sorted(to for to, _, _ in fake.copies())
+    assert len(places) == 4
+    n = fake.L.sb_field_size(h, fake.field(name))
+    fake.clear()
+    assert fake.L.sb_upload_field(h, fake.field(name), dp(a), n) == 0
+    copies = fake.copies()
+    assert copies
+    for to, _, size in copies:
+        assert not any(to < p < to + size for p in places)
+    fake.L.sb_destroy(h)
