@@ -402,7 +402,13 @@ int reset_bimocq(sb_bubble* b, const SbRestart& src = {}) {
     return SB_OK;
 }
 
-int upload_f32(sb_bubble* b, float* dst, const double* src, size_t n) {
+// Ends an upload: the caller's arrays are free again, whatever its outcome.
+int drained(sb_bubble* b, int rc) {
+    const cudaError_t e = cudaStreamSynchronize(b->stream);
+    return rc == SB_OK && e != cudaSuccess ? cuda_fail(e, "upload sync") : rc;
+}
+
+int queue_f32(sb_bubble* b, float* dst, const double* src, size_t n) {
     // the air flow's arrays have one element more than a landing place may hold
     const size_t room = (size_t)b->g.N;
     for (size_t at = 0; at < n; at += room) {
@@ -413,8 +419,11 @@ int upload_f32(sb_bubble* b, float* dst, const double* src, size_t n) {
                                   kStoreF32, b->stream));
         b->launches += 1;
     }
-    SB_CHECK(cudaStreamSynchronize(b->stream));
     return SB_OK;
+}
+
+int upload_f32(sb_bubble* b, float* dst, const double* src, size_t n) {
+    return drained(b, queue_f32(b, dst, src, n));
 }
 
 // Device FP32 staging for stored fields: the re-initialisation error
@@ -468,13 +477,16 @@ int set_base(sb_bubble* b, bool gamma, const double* v, size_t n) {
     return SB_OK;
 }
 
-int upload_scalar(sb_bubble* b, SbScalar* dst, const double* src, size_t n) {
+int queue_scalar(sb_bubble* b, SbScalar* dst, const double* src, size_t n) {
     int rc = copy_f64(b, 0, src, n);
     if (rc != SB_OK) return rc;
     SB_CHECK(launch_store_f64(dst, f64_buffer(b, 0), (int)n, base_of(b, dst), b->storage, b->stream));
     b->launches += 1;
-    SB_CHECK(cudaStreamSynchronize(b->stream));
     return SB_OK;
+}
+
+int upload_scalar(sb_bubble* b, SbScalar* dst, const double* src, size_t n) {
+    return drained(b, queue_scalar(b, dst, src, n));
 }
 
 int fill_const(sb_bubble* b, SbScalar* dst, size_t n, float v) {
@@ -938,11 +950,7 @@ int sb_upload_fields(sb_bubble* b, const double* eta, const double* gamma, const
             *in[k].to = f64_buffer(b, k);
         }
     if (rc == SB_OK) rc = reset_bimocq(b, src);
-    if (rc == SB_OK) {
-        cudaError_t e = cudaStreamSynchronize(b->stream);
-        if (e != cudaSuccess) rc = cuda_fail(e, "upload sync");
-    }
-    return rc;
+    return drained(b, rc);
 }
 
 }  // extern "C"

@@ -79,7 +79,7 @@ std::vector<Call> g_calls;
 extern "C" {
 
 // -- what the tests ask ------------------------------------------------------
-void fake_clear(void) { g_log.clear(); g_fail.clear(); }
+void fake_clear(void) { g_log.clear(); g_fail.clear(); g_error = cudaSuccess; }
 int fake_log_size(void) { return (int)g_log.size(); }
 const char* fake_log(int i) { return g_log[i].c_str(); }
 void fake_fail(const char* name, int nth) { g_fail[name] = nth; }  // the nth next call (once)

@@ -98,3 +98,29 @@ def test_uploads_stay_inside_their_landing_place(fake, nT, name):
     for to, _, size in copies:
         assert not any(to < p < to + size for p in places)
     fake.L.sb_destroy(h)
+
+
+@pytest.mark.parametrize("call,nth", [("cudaMemcpyAsync", 2), ("cudaMemcpyAsync", 4), ("launch", 1)])
+def test_a_failed_upload_leaves_no_copy_in_flight(fake, call, nth):
+    """The caller may free its arrays as soon as an upload has returned, also
+    with an error: every copy from them has been waited for."""
+    h = fake.bubble(64)
+    N = 2 * 64 * 64
+    a = np.zeros(N + 1)
+
+    def waited_for():
+        log = fake.log()
+        last = max((k for k, l in enumerate(log) if l.startswith("copy")), default=-1)
+        return "synchronised" in log[last + 1:]
+
+    fake.clear()
+    fake.fail(call, nth)
+    assert fake.L.sb_upload_fields(h, dp(a), dp(a), dp(a), dp(a), None, None) == fake.m.SB_ERR_CUDA
+    assert fake.log("failed") and waited_for()
+    for name in ("u_phi", "eta"):
+        fake.clear()
+        fake.fail(call, 1)
+        rc = fake.L.sb_upload_field(h, fake.field(name), dp(a), N)
+        assert rc == fake.m.SB_ERR_CUDA and waited_for()
+    fake.clear()
+    fake.L.sb_destroy(h)
