@@ -962,21 +962,10 @@ namespace {
 // unchanged step after step.
 int capture_plan(const SbStepPlan& P, cudaStream_t s, cudaGraphExec_t* out) {
     cudaGraph_t graph = nullptr;
-    // a second stream for the capture's branch (it ends with the capture)
-    cudaStream_t side = nullptr;
-    cudaEvent_t fork = nullptr, join = nullptr;
-    cudaError_t e = cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&fork, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&join, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
-    if (e == cudaSuccess) {
-        e = launch_plan_step(P, s, side, fork, join);
-        const cudaError_t e2 = cudaStreamEndCapture(s, &graph);
-        if (e == cudaSuccess) e = e2;
-    }
-    if (join) cudaEventDestroy(join);
-    if (fork) cudaEventDestroy(fork);
-    if (side) cudaStreamDestroy(side);
+    SB_CHECK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+    cudaError_t e = capture_plan_step(P, s);
+    const cudaError_t e2 = cudaStreamEndCapture(s, &graph);
+    if (e == cudaSuccess) e = e2;
     if (e == cudaSuccess) e = cudaGraphInstantiate(out, graph, 0);
     if (graph) cudaGraphDestroy(graph);
     if (e != cudaSuccess) return cuda_fail(e, "step graph capture");

@@ -227,14 +227,14 @@ struct SbStepPlan {
 
 // Occupancy queries and kernel attributes; call before any stream capture.
 cudaError_t prepare_plan(const SbStepPlan& P);
-// One stage of a step, the map-parity flip that ends a step, or the whole step.
+// One stage of a step, or the map-parity flip that ends a step.
 cudaError_t launch_plan_stage(const SbStepPlan& P, int stage, cudaStream_t s);
 // A map, velocity, thickness or accumulation stage of the members that the
 // chain kernels serve (sb_chain.cu).
 void launch_chain_stage(const SbStepPlan& P, int stage, cudaStream_t s);
 cudaError_t launch_plan_flip(const SbStepPlan& P, cudaStream_t s);
-cudaError_t launch_plan_step(const SbStepPlan& P, cudaStream_t s, cudaStream_t side, cudaEvent_t fork,
-                             cudaEvent_t join);
+// The whole step on a stream that is being captured.
+cudaError_t capture_plan_step(const SbStepPlan& P, cudaStream_t s);
 // Self-test of the bounded grid barrier on a bubble's barrier word (`blocks`
 // co-resident blocks, block `absent` never arrives; sb_step.cu).
 cudaError_t launch_barrier_probe(SbBubbleDesc* d, int blocks, int absent, unsigned limit,

@@ -21,6 +21,7 @@
 // bubble.cu:2633-2638) and is folded out.
 
 #include <algorithm>
+#include <vector>
 
 #include "sb_cells.cuh"
 #include "sb_internal.h"
@@ -1264,17 +1265,41 @@ cudaError_t launch_plan_flip(const SbStepPlan& P, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_plan_step(const SbStepPlan& P, cudaStream_t s, cudaStream_t side, cudaEvent_t fork,
-                             cudaEvent_t join) {
+namespace {
+
+// The nodes that the next launch captured on s waits for.
+cudaError_t capture_front(cudaStream_t s, std::vector<cudaGraphNode_t>& front) {
+    cudaStreamCaptureStatus status;
+    const cudaGraphNode_t* nodes = nullptr;
+    const cudaGraphEdgeData* edges = nullptr;
+    size_t n = 0;
+    const cudaError_t e = cudaStreamGetCaptureInfo(s, &status, nullptr, nullptr, &nodes, &edges, &n);
+    if (e != cudaSuccess) return e;
+    front.assign(nodes, nodes + n);
+    return cudaSuccess;
+}
+
+// `how`: cudaStreamSetCaptureDependencies or cudaStreamAddCaptureDependencies.
+cudaError_t wait_for(cudaStream_t s, std::vector<cudaGraphNode_t>& front, unsigned how) {
+    return cudaStreamUpdateCaptureDependencies(s, front.data(), nullptr, front.size(), how);
+}
+
+}  // namespace
+
+cudaError_t capture_plan_step(const SbStepPlan& P, cudaStream_t s) {
     // the velocities need nothing of the map and thickness stages: a branch of
-    // the captured step beside them, until the assembly
-    cudaError_t e = cudaEventRecord(fork, s);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(side, fork, 0);
+    // the captured step beside them, until the assembly (a second stream with
+    // events for it took 30 us of a new handle's first step)
+    std::vector<cudaGraphNode_t> start, maps, velocity;
+    cudaError_t e = capture_front(s, start);
     if (e == cudaSuccess) e = launch_plan_stage(P, STAGE_MAPS, s);
-    if (e == cudaSuccess) e = launch_plan_stage(P, STAGE_VELOCITY, side);
-    if (e == cudaSuccess) e = cudaEventRecord(join, side);
+    if (e == cudaSuccess) e = capture_front(s, maps);
+    if (e == cudaSuccess) e = wait_for(s, start, cudaStreamSetCaptureDependencies);
+    if (e == cudaSuccess) e = launch_plan_stage(P, STAGE_VELOCITY, s);
+    if (e == cudaSuccess) e = capture_front(s, velocity);
+    if (e == cudaSuccess) e = wait_for(s, maps, cudaStreamSetCaptureDependencies);
     if (e == cudaSuccess) e = launch_plan_stage(P, STAGE_BIMOCQ, s);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(s, join, 0);
+    if (e == cudaSuccess) e = wait_for(s, velocity, cudaStreamAddCaptureDependencies);
     for (int st = STAGE_ASSEMBLE; st < STAGE_COUNT && e == cudaSuccess; ++st) e = launch_plan_stage(P, st, s);
     return e == cudaSuccess ? launch_plan_flip(P, s) : e;
 }

@@ -124,3 +124,35 @@ def test_a_failed_upload_leaves_no_copy_in_flight(fake, call, nth):
         assert rc == fake.m.SB_ERR_CUDA and waited_for()
     fake.clear()
     fake.L.sb_destroy(h)
+
+
+@pytest.mark.parametrize("nT", [64, 1024])
+def test_a_captured_step_makes_no_streams_or_events(fake, nT):
+    """The first step of a handle or a batch captures its launches; the branch
+    of the velocities beside maps and thickness is made of the capture's own
+    dependencies, not of a stream and events made for it."""
+    h = fake.bubble(nT)
+    B = fake.batch([h])
+    for step in (lambda: fake.L.sb_batch_step(B, 1, 0.0, 0.005), lambda: fake.L.sb_step(h, 1, 0.0, 0.005)):
+        fake.clear()
+        assert step() == 0, fake.L.sb_last_error()
+        assert not fake.log("stream created") and not fake.log("event created")
+        nodes = [fake.L.fake_graph_node(i).decode() for i in range(fake.L.fake_graph_size())]
+        deps = [[int(d) for d in n.split(":")[1].split()] for n in nodes]
+        at = {k: i for k in ("advect_maps", "velocity", "bimocq", "assemble") for i, n in enumerate(nodes) if k in n}
+        assert len(nodes) == 9
+        assert deps[at["advect_maps"]] == deps[at["velocity"]] == []
+        assert deps[at["bimocq"]] == [at["advect_maps"]]
+        assert sorted(deps[at["assemble"]]) == sorted([at["velocity"], at["bimocq"]])
+        assert all(deps[i] == [i - 1] for i in range(at["assemble"] + 1, 9))
+    # a capture that fails leaves the handle usable
+    fake.clear()
+    g = fake.bubble(nT)
+    fake.fail("cudaStreamUpdateCaptureDependencies", 2)
+    assert fake.L.sb_step(g, 1, 0.0, 0.005) == fake.m.SB_ERR_CUDA
+    fake.clear()
+    assert fake.L.sb_step(g, 1, 0.0, 0.005) == 0
+    assert len(fake.log("launch")) == 9
+    fake.L.sb_batch_destroy(B)
+    fake.L.sb_destroy(h)
+    fake.L.sb_destroy(g)
