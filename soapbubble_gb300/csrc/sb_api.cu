@@ -1480,8 +1480,8 @@ struct sb_batch {
     cudaStream_t stream = nullptr;
     char* arena = nullptr;
     SbStepPlan plan{};  // the members as one set: their own descriptors, tiles, solve set
-    SbStepParams* h_params = nullptr;  // every member's step scalars, pinned
-    SbStepParams* d_params = nullptr;  // and on the device
+    std::vector<SbStepParams> h_params;  // every member's step scalars
+    SbStepParams* d_params = nullptr;    // and on the device
     cudaGraphExec_t graph = nullptr;
     cudaEvent_t ev[STAGE_COUNT + 1] = {};
     long long steps = 0;
@@ -1497,14 +1497,14 @@ int batch_set_params_each(sb_batch* B, const double* t, double dt) {
     for (size_t k = 0; k < B->m.size() && same; ++k)
         same = B->m[k]->last_t == t[k] && B->m[k]->last_dt == dt;
     if (same) return SB_OK;
-    SB_CHECK(cudaStreamSynchronize(B->stream));  // the pinned array may be in flight
     for (size_t k = 0; k < B->m.size(); ++k) {
-        step_params(B->m[k], t[k], dt, B->h_params + k);
+        step_params(B->m[k], t[k], dt, &B->h_params[k]);
         B->m[k]->last_dt = dt;
         B->m[k]->last_t = t[k];
     }
-    // one copy and one kernel for all members
-    SB_CHECK(cudaMemcpyAsync(B->d_params, B->h_params, sizeof(SbStepParams) * B->m.size(),
+    // one copy (from pageable memory: it has left the array when the call
+    // returns) and one kernel for all members
+    SB_CHECK(cudaMemcpyAsync(B->d_params, B->h_params.data(), sizeof(SbStepParams) * B->m.size(),
                              cudaMemcpyHostToDevice, B->stream));
     SB_CHECK(launch_set_params(B->plan.descs, B->d_params, (int)B->m.size(), B->stream));
     return SB_OK;
@@ -1612,18 +1612,21 @@ int sb_batch_create(sb_bubble* const* bubbles, int n, sb_batch** out) {
                  o_bar = L.take(sizeof(unsigned) * kGridBarWords),
                  o_params = L.take(sizeof(SbStepParams) * n);
     e = cudaMalloc((void**)&B->arena, L.bytes);
-    if (e == cudaSuccess) e = cudaMallocHost((void**)&B->h_params, sizeof(SbStepParams) * n);
-    if (e == cudaSuccess) e = cudaMemset(B->arena, 0, L.bytes);
     if (e != cudaSuccess) {
         int r = cuda_fail(e, "sb_batch_create allocation");
         sb_batch_destroy(B);
         return r;
     }
     char* A = B->arena;
+    // the arena's contents go up in one copy: the tables below, zeros elsewhere
+    std::vector<char> image(L.bytes, 0);
     // the members' own descriptors: a member keeps one map parity whether it
     // is stepped alone or here
-    std::vector<SbBubbleDesc*> descs(n);
-    for (int k = 0; k < n; ++k) descs[k] = B->m[k]->f.self;
+    for (int k = 0; k < n; ++k)
+        std::memcpy(&image[o_desc + k * sizeof(SbBubbleDesc*)], &B->m[k]->f.self, sizeof(SbBubbleDesc*));
+    for (int s = 0; s < 3; ++s)
+        std::memcpy(&image[o_tiles[s]], tiles[s].data(), sizeof(int2) * tiles[s].size());
+    std::memcpy(&image[o_roff], roff.data(), sizeof(int) * (n + 1));
     P.descs = (SbBubbleDesc* const*)(A + o_desc);
     P.nb = n;
     for (int s = 0; s < 3; ++s) {
@@ -1642,19 +1645,15 @@ int sb_batch_create(sb_bubble* const* bubbles, int n, sb_batch** out) {
     S.cnt = (int*)(A + o_cnt);
     S.acc = (unsigned long long*)(A + o_acc);
     S.bar = (unsigned*)(A + o_bar);
+    B->h_params.resize((size_t)n);
     B->d_params = (SbStepParams*)(A + o_params);
     // members may have work queued on their own streams; a member retired
     // from an earlier batch takes part again
     for (sb_bubble* b : B->m) e = e == cudaSuccess ? cudaStreamSynchronize(b->stream) : e;
     for (sb_bubble* b : B->m)
-        if (e == cudaSuccess) e = cudaMemset(&b->f.self->halted, 0, sizeof(int));
+        if (e == cudaSuccess) e = cudaMemsetAsync(&b->f.self->halted, 0, sizeof(int), B->stream);
     if (e == cudaSuccess)
-        e = cudaMemcpy((void*)P.descs, descs.data(), sizeof(SbBubbleDesc*) * n, cudaMemcpyHostToDevice);
-    for (int s = 0; s < 3 && e == cudaSuccess; ++s)
-        e = cudaMemcpy((void*)P.tiles[s], tiles[s].data(), sizeof(int2) * tiles[s].size(),
-                       cudaMemcpyHostToDevice);
-    if (e == cudaSuccess)
-        e = cudaMemcpy((void*)S.roff, roff.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice);
+        e = cudaMemcpyAsync(A, image.data(), image.size(), cudaMemcpyHostToDevice, B->stream);
     if (e != cudaSuccess) {
         int r = cuda_fail(e, "sb_batch_create upload");
         sb_batch_destroy(B);
@@ -1672,7 +1671,6 @@ int sb_batch_destroy(sb_batch* B) {
     for (cudaEvent_t e : B->ev)
         if (e) cudaEventDestroy(e);
     if (B->arena) cudaFree(B->arena);
-    if (B->h_params) cudaFreeHost(B->h_params);
     if (B->stream) cudaStreamDestroy(B->stream);
     delete B;
     return SB_OK;

@@ -150,9 +150,14 @@ cudaError_t cudaMalloc(void** p, size_t n) {
     return posix_memalign(p, 256, n ? n : 1) ? cudaErrorMemoryAllocation : cudaSuccess;
 }
 cudaError_t cudaFree(void* p) { free(p); return cudaSuccess; }
-cudaError_t cudaMallocHost(void** p, size_t n) { *p = malloc(n); return cudaSuccess; }
+cudaError_t cudaMallocHost(void** p, size_t n) {
+    note("page-locked");
+    *p = malloc(n);
+    return cudaSuccess;
+}
 cudaError_t cudaFreeHost(void* p) { free(p); return cudaSuccess; }
 cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) {
+    note("blocking copy");
     memcpy(d, s, n);
     return cudaSuccess;
 }
@@ -162,7 +167,11 @@ cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cu
     memcpy(d, s, n);
     return cudaSuccess;
 }
-cudaError_t cudaMemset(void* d, int v, size_t n) { memset(d, v, n); return cudaSuccess; }
+cudaError_t cudaMemset(void* d, int v, size_t n) {
+    note("blocking set");
+    memset(d, v, n);
+    return cudaSuccess;
+}
 cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t) {
     memset(d, v, n);
     return cudaSuccess;

@@ -156,3 +156,24 @@ def test_a_captured_step_makes_no_streams_or_events(fake, nT):
     fake.L.sb_batch_destroy(B)
     fake.L.sb_destroy(h)
     fake.L.sb_destroy(g)
+
+
+def test_a_batch_is_made_and_fed_without_pinning_or_blocking(fake):
+    """A serving loop rebuilds its batch whenever requests join: the tables go
+    up in one copy on the batch's own stream, and so do the step scalars."""
+    members = [fake.bubble(n) for n in (64, 128, 64)]
+    fake.clear()
+    B = fake.batch(members)
+    assert not fake.log("page-locked") and not fake.log("blocking")
+    assert len(fake.log("copy")) == 1
+    for t in ([0.1, 0.2, 0.3], [0.2, 0.2, 0.4]):
+        fake.clear()
+        ts = np.array(t)
+        assert fake.L.sb_batch_step_each(B, 1, dp(ts), 0.005) == 0
+        assert len(fake.log("copy")) == 1 and not fake.log("synchronised")
+    fake.clear()
+    assert fake.L.sb_batch_step_each(B, 1, dp(ts), 0.005) == 0
+    assert not fake.log("copy")  # unchanged
+    fake.L.sb_batch_destroy(B)
+    for m in members:
+        fake.L.sb_destroy(m)
