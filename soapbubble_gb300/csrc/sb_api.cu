@@ -1497,16 +1497,16 @@ int batch_set_params_each(sb_batch* B, const double* t, double dt) {
     for (size_t k = 0; k < B->m.size() && same; ++k)
         same = B->m[k]->last_t == t[k] && B->m[k]->last_dt == dt;
     if (same) return SB_OK;
-    for (size_t k = 0; k < B->m.size(); ++k) {
-        step_params(B->m[k], t[k], dt, &B->h_params[k]);
-        B->m[k]->last_dt = dt;
-        B->m[k]->last_t = t[k];
-    }
+    for (size_t k = 0; k < B->m.size(); ++k) step_params(B->m[k], t[k], dt, &B->h_params[k]);
     // one copy (from pageable memory: it has left the array when the call
     // returns) and one kernel for all members
     SB_CHECK(cudaMemcpyAsync(B->d_params, B->h_params.data(), sizeof(SbStepParams) * B->m.size(),
                              cudaMemcpyHostToDevice, B->stream));
     SB_CHECK(launch_set_params(B->plan.descs, B->d_params, (int)B->m.size(), B->stream));
+    for (size_t k = 0; k < B->m.size(); ++k) {
+        B->m[k]->last_dt = dt;
+        B->m[k]->last_t = t[k];
+    }
     return SB_OK;
 }
 

@@ -177,3 +177,20 @@ def test_a_batch_is_made_and_fed_without_pinning_or_blocking(fake):
     fake.L.sb_batch_destroy(B)
     for m in members:
         fake.L.sb_destroy(m)
+
+
+@pytest.mark.parametrize("call", ["cudaMemcpyAsync", "launch"])
+def test_step_scalars_that_did_not_arrive_are_sent_again(fake, call):
+    """A batch step whose scalars could not be sent leaves the members' frame
+    time unknown: the next call with the same time sends them."""
+    h = fake.bubble(64)
+    B = fake.batch([h])
+    assert fake.L.sb_batch_step(B, 1, 0.0, 0.005) == 0
+    fake.clear()
+    fake.fail(call, 1)
+    assert fake.L.sb_batch_step(B, 1, 0.5, 0.005) == fake.m.SB_ERR_CUDA
+    fake.clear()
+    assert fake.L.sb_batch_step(B, 1, 0.5, 0.005) == 0
+    assert len(fake.log("copy")) == 1 and any("k_set_params" in l for l in fake.log("launch"))
+    fake.L.sb_batch_destroy(B)
+    fake.L.sb_destroy(h)
