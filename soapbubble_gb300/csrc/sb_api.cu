@@ -1506,6 +1506,7 @@ int batch_set_params_each(sb_batch* B, const double* t, double dt) {
     for (size_t k = 0; k < B->m.size(); ++k) {
         B->m[k]->last_dt = dt;
         B->m[k]->last_t = t[k];
+        B->m[k]->launches += 1;  // k_set_params
     }
     return SB_OK;
 }

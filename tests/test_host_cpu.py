@@ -194,3 +194,24 @@ def test_step_scalars_that_did_not_arrive_are_sent_again(fake, call):
     assert len(fake.log("copy")) == 1 and any("k_set_params" in l for l in fake.log("launch"))
     fake.L.sb_batch_destroy(B)
     fake.L.sb_destroy(h)
+
+
+def test_launch_counts_include_the_step_scalars(fake):
+    """sb_stats.launches counts the kernels that served a handle: a batch of
+    one counts what the runtime saw."""
+    h = fake.bubble(64)
+    B = fake.batch([h])
+    st = fake.m.SbStats()
+
+    def count():
+        assert fake.L.sb_get_stats(h, C.byref(st)) == 0
+        return st.launches
+
+    before = count()
+    fake.clear()
+    for t in (0.1, 0.1, 0.2):
+        assert fake.L.sb_batch_step(B, 2, t, 0.005) == 0
+    assert len(fake.log("launch")) == 3 * 2 * 9 + 2
+    assert count() - before == len(fake.log("launch"))
+    fake.L.sb_batch_destroy(B)
+    fake.L.sb_destroy(h)
