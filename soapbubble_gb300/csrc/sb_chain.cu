@@ -353,6 +353,7 @@ __global__ void __launch_bounds__(256 * PAR, PAR == 1 ? 5 : 2) k_velocity_chains
 }
 
 constexpr int kSampleCells = 64;  // cells of a block with its samples in parallel
+static_assert(kSampleCells == kTileSizes[0], "launched over the smallest tiles");
 
 // PAR = 1: the tile's cells, one per thread; PAR = 5: a pair of warps per
 // sample point; the first pair adds the samples up in their order.
@@ -570,7 +571,6 @@ void launch_chains(const SbStepPlan& P, int tile, int par, K* one, K* each, cuda
 void launch_chain_stage(const SbStepPlan& P, int stage, cudaStream_t s) {
     const int k = P.sel[stage];
     const bool par = P.nchain[0] * kTileSizes[0] <= kChipThreads;
-    static_assert(kSampleCells == 64, "the smallest tile");
     switch (stage) {
         case STAGE_MAPS:
             if (par) launch_chains(P, k, 2, k_advect_maps_chains<true, 2>, k_advect_maps_chains<false, 2>, s);

@@ -204,7 +204,7 @@ cudaError_t launch_solve_one(const SbGrid& g, const SbFields& f, const SbSolveSe
                              const SolverConfig& cfg, cudaStream_t s);
 
 // Cells per block of the three tile sizes the stage kernels can use.
-extern const int kTileSizes[3];
+constexpr int kTileSizes[3] = {64, 128, 256};
 
 // Everything one step launches over a set of bubbles (one bubble, or every
 // bubble of a batch; sb_step.cu).  Device arrays: descs[k] points to bubble

@@ -1187,8 +1187,6 @@ int reinit_blocks() {
 
 }  // namespace
 
-const int kTileSizes[3] = {64, 128, 256};
-
 cudaError_t prepare_plan(const SbStepPlan& P) {
     reinit_blocks();
     return prepare_solve(P.maxNP, P.solver, nullptr);

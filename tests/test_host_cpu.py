@@ -215,3 +215,22 @@ def test_launch_counts_include_the_step_scalars(fake):
     assert count() - before == len(fake.log("launch"))
     fake.L.sb_batch_destroy(B)
     fake.L.sb_destroy(h)
+
+
+def test_a_smaller_smallest_tile_does_not_compile(tmp_path):
+    """The parallel chain kernels deal kSampleCells cells to a block and are
+    launched over the smallest tiles: another smallest tile is refused when
+    they are compiled, and does not index out of their shared arrays."""
+    import shutil
+    from soapbubble_gb300 import build
+    src = tmp_path / "csrc"
+    shutil.copytree(build.CSRC, src)
+    for f in src.iterdir():
+        t = f.read_text()
+        f.write_text(t.replace("kTileSizes[3] = {64, 128, 256}", "kTileSizes[3] = {32, 128, 256}"))
+    cmd = [build.nvcc(), "-gencode", "arch=compute_103a,code=sm_103a", "-std=c++17", "--expt-relaxed-constexpr",
+           "-I", os.path.join(build.ROOT, "include"), "-I", str(src), "--cuda", str(src / "sb_chain.cu"),
+           "-o", str(tmp_path / "out.ii")]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    assert r.returncode != 0
+    assert "static assertion" in r.stdout + r.stderr
