@@ -1009,7 +1009,7 @@ int autotune_plan(SbStepPlan& P, StepFn step, int* tile_sizes) {
         for (int k = 0; k < 3; ++k)
             if (ms[k][st] < ms[best][st]) best = k;
         P.sel[st] = best;
-        if (tile_sizes) tile_sizes[st] = kTileSizes[best];
+        if (tile_sizes) tile_sizes[st] = kTileSizes[stage_tile(P, st)];
     }
     return SB_OK;
 }

@@ -560,6 +560,8 @@ namespace {
 // (512 x 1024: k_bimocq 49 us against 58, k_accum 39 against 53).
 constexpr int kChipThreads = 152 * 1024;
 
+bool parallel_chains(const SbStepPlan& P) { return P.nchain[0] * kTileSizes[0] <= kChipThreads; }
+
 // PAR chains of a cell in parallel over the set's tiles of size tile.
 template <class K>
 void launch_chains(const SbStepPlan& P, int tile, int par, K* one, K* each, cudaStream_t s) {
@@ -568,9 +570,15 @@ void launch_chains(const SbStepPlan& P, int tile, int par, K* one, K* each, cuda
 
 }  // namespace
 
+int stage_tile(const SbStepPlan& P, int stage) {
+    const bool fixed = parallel_chains(P) && P.nchain[0] == P.ntiles[0] &&
+                       (stage == STAGE_BIMOCQ || stage == STAGE_ACCUM);
+    return fixed ? 0 : P.sel[stage];
+}
+
 void launch_chain_stage(const SbStepPlan& P, int stage, cudaStream_t s) {
     const int k = P.sel[stage];
-    const bool par = P.nchain[0] * kTileSizes[0] <= kChipThreads;
+    const bool par = parallel_chains(P);
     switch (stage) {
         case STAGE_MAPS:
             if (par) launch_chains(P, k, 2, k_advect_maps_chains<true, 2>, k_advect_maps_chains<false, 2>, s);

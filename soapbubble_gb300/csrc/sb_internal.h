@@ -232,6 +232,8 @@ cudaError_t launch_plan_stage(const SbStepPlan& P, int stage, cudaStream_t s);
 // A map, velocity, thickness or accumulation stage of the members that the
 // chain kernels serve (sb_chain.cu).
 void launch_chain_stage(const SbStepPlan& P, int stage, cudaStream_t s);
+// The tile size (index into kTileSizes) that a stage of the plan uses.
+int stage_tile(const SbStepPlan& P, int stage);
 cudaError_t launch_plan_flip(const SbStepPlan& P, cudaStream_t s);
 // The whole step on a stream that is being captured.
 cudaError_t capture_plan_step(const SbStepPlan& P, cudaStream_t s);

@@ -234,3 +234,26 @@ def test_a_smaller_smallest_tile_does_not_compile(tmp_path):
     r = subprocess.run(cmd, capture_output=True, text=True)
     assert r.returncode != 0
     assert "static assertion" in r.stdout + r.stderr
+
+
+@pytest.mark.parametrize("sizes,kw,fixed", [([64], {}, True), ([64, 64], {}, True), ([512], {}, False),
+                                            ([64], {"storage": 1}, False), ([64, 1024], {}, False)])
+def test_autotune_reports_the_tiles_in_use(fake, sizes, kw, fixed):
+    """Small FP32 sets sample thickness and accumulation over 64-cell tiles
+    whatever was timed; the sizes reported are the sizes used (the fake
+    runtime times every size alike, which selects 128)."""
+    members = [fake.bubble(n, **kw) for n in sizes]
+    out = (C.c_int * 8)()
+    if len(members) == 1:
+        assert fake.L.sb_autotune(members[0], 0.0, 0.005, out) == 0
+    else:
+        B = fake.batch(members)
+        assert fake.L.sb_batch_autotune(B, 0.0, 0.005, out) == 0
+        fake.L.sb_batch_destroy(B)
+    names = [fake.L.sb_stage_name(k).decode() for k in range(8)]
+    got = dict(zip(names, out))
+    want = 64 if fixed else 128
+    assert got["k_bimocq"] == got["k_accum"] == want
+    assert got["k_advect_maps"] == got["k_assemble"] == 128
+    for m in members:
+        fake.L.sb_destroy(m)
