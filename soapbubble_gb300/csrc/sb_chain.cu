@@ -553,14 +553,17 @@ __global__ void __launch_bounds__(PAR == 1 ? 256 : 6 * kSampleCells, 4) k_accum_
 namespace {
 
 // A set's cells decide the form.  Below one thread per cell of a full chip
-// (152 SMs x 1024 threads) the chains run in parallel: there a launch lasts as
+// (1024 threads an SM, 155,648 on 152 SMs) the chains run in parallel: there a launch lasts as
 // long as its longest thread (64 x 128: 40 us per step against 47; 256 x 512:
 // k_bimocq 22 us against 33, k_velocity 14 against 16).  Above it they run in
 // one thread, which shares the five-point lookups and needs no exchange
 // (512 x 1024: k_bimocq 49 us against 58, k_accum 39 against 53).
-constexpr int kChipThreads = 152 * 1024;
-
-bool parallel_chains(const SbStepPlan& P) { return P.nchain[0] * kTileSizes[0] <= kChipThreads; }
+bool parallel_chains(const SbStepPlan& P) {
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return P.nchain[0] * kTileSizes[0] <= sms * 1024;
+}
 
 // PAR chains of a cell in parallel over the set's tiles of size tile.
 template <class K>

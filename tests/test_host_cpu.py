@@ -257,3 +257,23 @@ def test_autotune_reports_the_tiles_in_use(fake, sizes, kw, fixed):
     assert got["k_advect_maps"] == got["k_assemble"] == 128
     for m in members:
         fake.L.sb_destroy(m)
+
+
+def test_the_chains_are_dealt_by_the_device_at_hand(fake):
+    """Chains run in parallel below one thread per cell of the device, of
+    however many multiprocessors it has."""
+    def form(nT):
+        h = fake.bubble(nT)
+        fake.clear()
+        assert fake.L.sb_step(h, 1, 0.0, 0.005) == 0
+        names = [l for l in fake.log("launch") if "k_bimocq_chains" in l]
+        fake.L.sb_destroy(h)
+        assert len(names) == 1
+        return int(names[0].split("Li")[1].split("E")[0])  # the kernel's PAR argument
+
+    try:
+        assert [form(n) for n in (64, 256, 512)] == [5, 5, 1]
+        fake.L.fake_set_sms(8)
+        assert [form(n) for n in (64, 128, 256)] == [5, 1, 1]
+    finally:
+        fake.L.fake_set_sms(152)
