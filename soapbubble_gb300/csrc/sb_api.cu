@@ -388,7 +388,13 @@ double* f64_buffer(sb_bubble* b, int k) {
 
 // Uploads arrive in FP64 and are rounded on the device: the host's loops over
 // them took 0.25 ms of a 512 x 1024 field's 0.3, a page-locked or pageable
-// copy of the doubles takes 0.035 and the kernel 0.01.
+// copy of the doubles takes 0.035 and the kernel 0.01.  A small FP32 field by
+// itself is rounded on the host all the same, where the kernel and twice the
+// bytes cost more than the loop (u_phi, us, host / device: 64 x 128 16 / 20,
+// 128 x 256 23 / 26, 256 x 512 58 / 31); a stored field takes a kernel in any
+// case.
+constexpr size_t kHostRounded = 2 * 128 * 128 + 1;  // elements, with the air flow's last
+
 int copy_f64(sb_bubble* b, int k, const double* src, size_t n) {
     if (n > (size_t)b->g.N) return fail(SB_ERR_INVALID, "upload larger than its landing place");
     SB_CHECK(cudaMemcpyAsync(f64_buffer(b, k), src, n * sizeof(double), cudaMemcpyHostToDevice, b->stream));
@@ -408,7 +414,12 @@ int drained(sb_bubble* b, int rc) {
     return rc == SB_OK && e != cudaSuccess ? cuda_fail(e, "upload sync") : rc;
 }
 
-int queue_f32(sb_bubble* b, float* dst, const double* src, size_t n) {
+int queue_f32(sb_bubble* b, float* dst, const double* src, size_t n, std::vector<float>& rounded) {
+    if (n <= kHostRounded) {
+        rounded.assign(src, src + n);
+        SB_CHECK(cudaMemcpyAsync(dst, rounded.data(), n * sizeof(float), cudaMemcpyHostToDevice, b->stream));
+        return SB_OK;
+    }
     // the air flow's arrays have one element more than a landing place may hold
     const size_t room = (size_t)b->g.N;
     for (size_t at = 0; at < n; at += room) {
@@ -423,7 +434,8 @@ int queue_f32(sb_bubble* b, float* dst, const double* src, size_t n) {
 }
 
 int upload_f32(sb_bubble* b, float* dst, const double* src, size_t n) {
-    return drained(b, queue_f32(b, dst, src, n));
+    std::vector<float> rounded;  // until the stream has drained
+    return drained(b, queue_f32(b, dst, src, n, rounded));
 }
 
 // Device FP32 staging for stored fields: the re-initialisation error

@@ -104,8 +104,8 @@ def test_uploads_stay_inside_their_landing_place(fake, nT, name):
 def test_a_failed_upload_leaves_no_copy_in_flight(fake, call, nth):
     """The caller may free its arrays as soon as an upload has returned, also
     with an error: every copy from them has been waited for."""
-    h = fake.bubble(64)
-    N = 2 * 64 * 64
+    h = fake.bubble(256)
+    N = 2 * 256 * 256
     a = np.zeros(N + 1)
 
     def waited_for():
@@ -277,3 +277,15 @@ def test_the_chains_are_dealt_by_the_device_at_hand(fake):
         assert [form(n) for n in (64, 128, 256)] == [5, 1, 1]
     finally:
         fake.L.fake_set_sms(152)
+
+
+@pytest.mark.parametrize("nT,launches", [(16, 0), (128, 0), (256, 1)])
+def test_small_fields_take_one_copy_and_no_kernel(fake, nT, launches):
+    """FP32 arrays of up to 128 x 256 cells are rounded on the host: a kernel
+    behind the copy would take longer than the host's loop."""
+    h = fake.bubble(nT)
+    a = np.zeros(2 * nT * nT)
+    fake.clear()
+    assert fake.L.sb_upload_field(h, fake.field("u_phi"), dp(a), a.size) == 0
+    assert len(fake.log("copy")) == 1 and len(fake.log("launch")) == launches
+    fake.L.sb_destroy(h)
