@@ -74,7 +74,8 @@ __device__ __forceinline__ bool fast_departure(const SbBubbleDesc& d, int idx, f
     const float gp = 0.5f * f.uph[idx] + 0.5f * f.uph[(i << g.logP) + ((j + 1) & g.maskP)];
     FTrace T;
     FPos q;
-    bool ok = fast_trace<kAtCell, true>(g, f.uth, f.uph, i, j, F.s0, F.c0, gt, gp, dt, true, T);
+    bool ok = fast_trace<kAtCell, true>(g, f.uth, f.uph, i, j, F.s0, F.c0, gt, gp, dt, fast_rests(gt, gp),
+                                         true, T);
     ok &= fast_pos<true>(g, F.s0, F.c0, T.d, q);
     ok &= fast_stencil(g, i, j + q.flip, q.o, g.nT - 2, s);
     return ok;
@@ -159,10 +160,18 @@ __device__ __forceinline__ bool velocity_fast(const SbBubbleDesc& d, int idx, fl
         gt = f.uth[idx];
         gp = lerp4(f.uph[idx], f.uph[e], f.uph[idx + nP], f.uph[e + nP], dup(0.5f));
     }
+    // no trace to run: at rest the face keeps its speed, and beside a torn one
+    // (NaN) there is no fast form.  Two tests in this order: one for both and a
+    // second behind it took 23.9 us in place of 22.6 at 512 x 1024
+    if (fast_rests(gt, gp)) {
+        out = 0.0f;
+        return true;
+    }
+    if (!(fmaf(gt, gt, __fmul_rn(gp, gp)) > 1e-30f)) return false;
     FTrace T;
     FPos q;
     float vt, vp, a, n;
-    bool ok = fast_trace<KIND, false>(g, f.uth, f.uph, i, j, s0, c0, gt, gp, f.step->dt,
+    bool ok = fast_trace<KIND, false>(g, f.uth, f.uph, i, j, s0, c0, gt, gp, f.step->dt, false,
                                       !d.ph.single_step, T);
     ok &= fast_pos<false>(g, s0, c0, T.d, q);
     ok &= fast_velocity<KIND>(g, f.uth, f.uph, i, j + q.flip, q.o, vt, vp);
