@@ -1376,6 +1376,11 @@ k_solve(SbSolveSet S, SolverConfig cfg) {
     stage_init(St, &bar, sm, cfg.blob);
     const unsigned G = gridDim.x;
     const unsigned* const s_pre = H.pre;
+    // Every block has to see the same kinds, and a block that starts late may
+    // read statistics that a system finishing in phase 0 is writing.  Only one
+    // that starts with K_SETUP_L can finish there, with 0 iterations, and any
+    // mix of its old and new words says K_SETUP_L again.
+    static_assert(kNeumannOff < kNeumannOn, "a mix of old and new statistics could choose K_SETUP");
     for (int b = threadIdx.x; b < S.nb; b += TB) {
         const SbBubbleDesc* d = S.descs[b];
         H.rows[b] = d->halted ? 0 : (unsigned short)(S.roff[b + 1] - S.roff[b]);
