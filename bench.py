@@ -43,8 +43,10 @@ NTHETA, DT, RECIPE, SEED = 512, 0.002, "c1", 20261203
 STEPS_PER_FRAME = 10
 L2_FLUSH_BYTES = 512 << 20
 
-# Algorithmic bytes per cell and launch (every array a kernel must read or
-# write counted once; halo re-reads excluded)
+# Algorithmic bytes per cell and launch (every array that a stage of the
+# algorithm must read or write counted once; halo re-reads excluded, and so are
+# the words that the kernels add for themselves: 16 B written by k_post for
+# k_accum's samples, 16 B read and 12 B written by k_advect_maps for k_bimocq's)
 # (FP32 = 4 B, map entry = 16 B: a float4 displacement).
 ALG_BYTES_PER_CELL = {
     "k_advect_maps": 104,  # u_th,u_ph,fwd,bwd,gamma,uair0,corr_u,vair0,corr_v -> fwd',bwd',gamma',uair,vair

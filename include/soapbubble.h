@@ -228,13 +228,15 @@ int sb_step_timed(sb_bubble* b, int n_steps, double t_frame, double dt, double* 
 
 /* Picks, per stage, the tile size (64, 128 or 256 cells per block) with the
  * shortest device time, from one timed step at each size; tile_sizes
- * (optional, sb_stage_count() ints) receives the choice.  The three tuning
+ * (optional, sb_stage_count() ints) receives the size that each stage uses
+ * from then on (a stage that has one size only, as the sampling stages of
+ * small FP32 sets, reports that one).  The three tuning
  * steps advance the bubble like sb_step_timed.  Results do not depend on
  * the tile sizes.  No counterpart in the reference. */
 int sb_autotune(sb_bubble* b, double t_frame, double dt, int* tile_sizes);
 
 /* Number of kernel stages of one step, and the kernel name of a stage.  A
- * step launches one kernel per stage plus one that flips the map parity. */
+ * bubble's step is one kernel per stage plus one that flips the map parity. */
 int sb_stage_count(void);
 const char* sb_stage_name(int stage);
 
@@ -367,7 +369,9 @@ const char* sb_last_error(void);
 
 /* ------------------------------------------------------------------------
  * Batches: an ensemble of bubbles (any mix of grid sizes on one device)
- * stepped together, one kernel launch per stage for all members.
+ * stepped together, each stage launched over all members at once: one kernel
+ * for all, or, in the map, velocity, thickness and accumulation stages, one
+ * for the FP32 members of up to 512 rows and one for the others.
  *
  * The reference has no counterpart; it steps one Solver per process
  * (Bubble::run, kernel/bubble.cu:2607-2704).  A batch step gives every
@@ -389,7 +393,8 @@ typedef struct sb_batch sb_batch;
  * and 256 cells, solve-block ranges).  Synchronises the members' streams.
  * A bubble listed twice is rejected (SB_ERR_INVALID), and so is a batch
  * over its limits: at most 1024 members, and the sum over members of
- * nTheta (2 nTheta + 256) below 2^32 (the solver's 32-bit row tables). */
+ * nTheta (2 nTheta + 256) below 2^32 (an upper bound of the solver's 32-bit
+ * sums of row weights). */
 int sb_batch_create(sb_bubble* const* members, int n, sb_batch** out);
 int sb_batch_destroy(sb_batch* batch);
 

@@ -235,8 +235,8 @@ def batch_weight(nTheta: int) -> int:
 
 
 class GpuBatch:
-    """An ensemble of GpuBubbles stepped together (sb_batch_*): one kernel
-    launch per stage for all members, one CUDA graph per step.  The members
+    """An ensemble of GpuBubbles stepped together (sb_batch_*): each stage
+    launched over all members at once, one CUDA graph per step.  The members
     stay owned by the caller; step them only through the batch while it
     exists, and synchronize() before reading their fields."""
 

@@ -1482,7 +1482,7 @@ const char* sb_last_error(void) { return g_err.c_str(); }
 }  // extern "C"
 
 // ---------------------------------------------------------------------------
-// Batches: many bubbles stepped together, one launch per stage.
+// Batches: many bubbles stepped together, each stage launched over all of them.
 // ---------------------------------------------------------------------------
 
 struct sb_batch {
@@ -1583,7 +1583,8 @@ int sb_batch_create(sb_bubble* const* bubbles, int n, sb_batch** out) {
         B->retired.push_back(0);
         if (b->g.nP > P.maxNP) P.maxNP = b->g.nP;
     }
-    // the row list of the solve: every member's theta rows, member by member
+    // the row list of the solve: every member's theta rows, member by member;
+    // weight bounds the rows' weights of any phase (row_weight, sb_solver.cu)
     std::vector<int> roff(n + 1, 0);
     unsigned long long weight = 0;
     for (int k = 0; k < n; ++k) {

@@ -120,8 +120,10 @@ struct SolverConfig {
 };
 
 // Step stages in launch order (sb_step.cu, sb_solver.cu).  `cur` selects the
-// map ping-pong buffers.  Each stage is one kernel launch; a step ends with a
-// flip of every bubble's map parity (one more launch).
+// map ping-pong buffers.  A stage is one kernel launch for each kind of member
+// that the set holds (members that the chain kernels serve and others, in the
+// four stages that have chain kernels; one for all in the rest); a step ends
+// with a flip of every bubble's map parity (one more launch).
 enum SbStage {
     STAGE_MAPS = 0,   // k_advect_maps: characteristic maps, gamma, air flow
     STAGE_VELOCITY,   // k_velocity: u_theta / u_phi self-advection
@@ -177,8 +179,9 @@ constexpr int kSolveAccWords = 3 * 3 * 16;  // 3 buffers x 3 values x one 128-by
 constexpr int kGridBarWords = 32;           // grid barrier word on its own 128-byte line (sb_sync.cuh)
 
 // A set of implicit systems solved by one cooperative launch: the system of
-// one bubble, or the systems of every bubble of a batch (at most 1024, with
-// sum over systems of nT (2 nT + 256) below 2^32).  Device arrays.
+// one bubble, or the systems of every bubble of a batch: at most 1024, with
+// the sum over systems of nT (2 nT + 256) below 2^32, which bounds the sum of
+// the rows' weights in any phase (row_weight).  Device arrays.
 struct SbSolveSet {
     SbBubbleDesc* const* descs;  // [nb] device pointers to each bubble's descriptor
     int nb;

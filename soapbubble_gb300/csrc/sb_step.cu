@@ -589,8 +589,8 @@ __device__ __forceinline__ void assemble_quad(const SbGrid& g, const SbPhys& ph,
 
 // After the solve: divergence from gamma, friction/Marangoni/gravity velocity
 // update, thickness update with evaporation, and the per-step changes that
-// BIMOCQ accumulates.  Increments are carried directly (dx from the solve,
-// d_eta = -eta dt div + evap dt) instead of as differences of O(1) values.
+// BIMOCQ accumulates.  Increments are carried directly (dx from the solve, the
+// thickness's -eta dt div + evap dt) instead of as differences of O(1) values.
 // changes holds what the accumulation samples, the fields as they were stored.
 // Neighbouring new gamma values are clamped on the fly exactly as
 // divergenceKernel_fromGamma clamps them in place (kernel/bubble.cu:1287;
@@ -965,9 +965,8 @@ __device__ __forceinline__ int nb_index(const SbGrid& g, int i, int j) {
 
 // correctCentered2: subtract the error pulled back through the backward map,
 // clamp to the 3x3 range of the uncorrected field, keep non-negative.  The
-// result goes to the per-step increment buffers (read by k_accum, free from
-// here on; the *_adv buffers keep the step's implicit system) and is
-// committed in the next phase.
+// result goes to arrays of its own (d_eta, d_gam; the *_adv buffers keep the
+// step's implicit system) and is committed in the next phase.
 template <class T>
 __device__ __forceinline__ void reinit_correct(const SbGrid& g, const SbPhys& ph, const SbFields& f, int cur,
                                                int idx) {

@@ -5,7 +5,7 @@ blurred seeded 16 x 8 checkerboard, surfactant 1 + 0.05 SH(<= 16)).
 Both runs start from the same fields and take the same steps; each reports
 its device time per step (graph-launched steps between CUDA events; the
 state of ~480 MB is far above L2, so no flush is needed), its per-stage
-times with the algorithmic bytes each stage moves in that storage, and the
+times with the algorithmic bytes of each stage in that storage, and the
 BF16 run's difference from the FP32 run at the end.
 
     python -m soapbubble_gb300.storage [--steps 100]
@@ -20,8 +20,11 @@ import numpy as np
 from . import cudart, synth
 from .bubble import GpuBubble, bytes_required, make_params, stage_names
 
-# Algorithmic bytes per cell and launch (every array once; FP32 = 4 B, map
-# entry = 16 B, a stored field 4 or 2 B).  s = bytes of a stored element.
+# Algorithmic bytes per cell and launch: what each stage of the algorithm must
+# read and write, every array once (FP32 = 4 B, map entry = 16 B, a stored field
+# 4 or 2 B); s = bytes of a stored element.  The kernels move more: k_post writes
+# a 16-byte word of changes beside them, from which k_accum samples, and the
+# map kernels of FP32 grids up to 512 rows 12 bytes for the thickness stage.
 def alg_bytes(s: int) -> dict:
     return {
         "k_advect_maps": 100 + s,     # gamma sampled in the stored type; maps 16 B
