@@ -32,12 +32,17 @@ struct Event {
 std::vector<std::string> g_log;
 std::string g_line;
 std::map<std::string, int> g_fail;  // calls of a name until one fails
-std::map<const void*, std::string> g_kernels;
 Graph* g_capture = nullptr;  // the capture in progress
 std::vector<Stream*> g_captured_streams;
 std::vector<Node> g_last_graph;
 int g_sms = 152;
 cudaError_t g_error = cudaSuccess;
+
+// Filled while the library's objects are initialised, in whatever order.
+std::map<const void*, std::string>& kernels() {
+    static std::map<const void*, std::string> k;
+    return k;
+}
 
 void note(const std::string& s) { g_log.push_back(s); }
 std::string num(const void* p) { return std::to_string((unsigned long long)p); }
@@ -61,7 +66,7 @@ void captured(Stream* s, const std::string& kernel) {
 cudaError_t launch(const void* fn, cudaStream_t stream) {
     MAY_FAIL("launch");
     Stream* s = (Stream*)stream;
-    const std::string& k = g_kernels[fn];
+    const std::string& k = kernels()[fn];
     if (s && s->capturing) captured(s, k);
     else note("launch " + k);
     return cudaSuccess;
@@ -97,7 +102,7 @@ void __cudaRegisterFatBinaryEnd(void**) {}
 void __cudaUnregisterFatBinary(void**) {}
 void __cudaRegisterFunction(void**, const char* host, char*, const char* name, int, uint3*, uint3*,
                             dim3*, dim3*, int*) {
-    g_kernels[host] = name;
+    kernels()[host] = name;
 }
 void __cudaRegisterVar(void**, char*, char*, const char*, int, size_t, int, int) {}
 unsigned __cudaPushCallConfiguration(dim3 grid, dim3 block, size_t smem, cudaStream_t stream) {
