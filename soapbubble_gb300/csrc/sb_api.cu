@@ -1509,9 +1509,9 @@ int batch_set_params_each(sb_batch* B, const double* t, double dt) {
     for (size_t k = 0; k < B->m.size() && same; ++k)
         same = B->m[k]->last_t == t[k] && B->m[k]->last_dt == dt;
     if (same) return SB_OK;
+    SB_CHECK(cudaStreamSynchronize(B->stream));  // the scalars before may be in flight
     for (size_t k = 0; k < B->m.size(); ++k) step_params(B->m[k], t[k], dt, &B->h_params[k]);
-    // one copy (from pageable memory: it has left the array when the call
-    // returns) and one kernel for all members
+    // one copy and one kernel for all members
     SB_CHECK(cudaMemcpyAsync(B->d_params, B->h_params.data(), sizeof(SbStepParams) * B->m.size(),
                              cudaMemcpyHostToDevice, B->stream));
     SB_CHECK(launch_set_params(B->plan.descs, B->d_params, (int)B->m.size(), B->stream));
@@ -1668,6 +1668,7 @@ int sb_batch_create(sb_bubble* const* bubbles, int n, sb_batch** out) {
         if (e == cudaSuccess) e = cudaMemsetAsync(&b->f.self->halted, 0, sizeof(int), B->stream);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(A, image.data(), image.size(), cudaMemcpyHostToDevice, B->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(B->stream);
     if (e != cudaSuccess) {
         int r = cuda_fail(e, "sb_batch_create upload");
         sb_batch_destroy(B);
