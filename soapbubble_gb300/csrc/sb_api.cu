@@ -1605,20 +1605,14 @@ int sb_batch_create(sb_bubble* const* bubbles, int n, sb_batch** out) {
         sb_batch_destroy(B);
         return r;
     }
-    // tiles for the three tile sizes
-    std::vector<int2> tiles[3];
-    for (int s = 0; s < 3; ++s)
-        for (int chains = 1; chains >= 0; --chains) {  // the chain kernels' members first
-            for (int k = 0; k < n; ++k)
-                if (B->m[k]->desc.chains == chains)
-                    for (int c = 0; c < B->m[k]->g.N; c += kTileSizes[s])
-                        tiles[s].push_back(make_int2(k, c));
-            if (chains) P.nchain[s] = (int)tiles[s].size();
-        }
     Layout L;
     const size_t o_desc = L.take(sizeof(SbBubbleDesc*) * n);
     size_t o_tiles[3];
-    for (int s = 0; s < 3; ++s) o_tiles[s] = L.take(sizeof(int2) * tiles[s].size());
+    for (int s = 0; s < 3; ++s) {
+        P.ntiles[s] = 0;
+        for (const sb_bubble* b : B->m) P.ntiles[s] += (b->g.N + kTileSizes[s] - 1) / kTileSizes[s];
+        o_tiles[s] = L.take(sizeof(int2) * P.ntiles[s]);
+    }
     const size_t o_roff = L.take(sizeof(int) * (n + 1)),
                  o_rec = L.take(sizeof(SbSolveRec) * 2 * n), o_done = L.take(sizeof(int) * n),
                  o_cnt = L.take(sizeof(int) * n),
@@ -1632,21 +1626,28 @@ int sb_batch_create(sb_bubble* const* bubbles, int n, sb_batch** out) {
         return r;
     }
     char* A = B->arena;
-    // the arena's contents go up in one copy: the tables below, zeros elsewhere
-    std::vector<char> image(L.bytes, 0);
+    // the arena's contents go up in one copy: the tables, and zeros behind them
+    const std::unique_ptr<char[]> image(new char[L.bytes]);
     // the members' own descriptors: a member keeps one map parity whether it
     // is stepped alone or here
-    for (int k = 0; k < n; ++k)
-        std::memcpy(&image[o_desc + k * sizeof(SbBubbleDesc*)], &B->m[k]->f.self, sizeof(SbBubbleDesc*));
-    for (int s = 0; s < 3; ++s)
-        std::memcpy(&image[o_tiles[s]], tiles[s].data(), sizeof(int2) * tiles[s].size());
-    std::memcpy(&image[o_roff], roff.data(), sizeof(int) * (n + 1));
+    SbBubbleDesc** descs = (SbBubbleDesc**)(image.get() + o_desc);
+    for (int k = 0; k < n; ++k) descs[k] = B->m[k]->f.self;
+    // tiles for the three tile sizes, the chain kernels' members first
+    for (int s = 0; s < 3; ++s) {
+        int2* t = (int2*)(image.get() + o_tiles[s]);
+        const int2* const first = t;
+        for (int chains = 1; chains >= 0; --chains) {
+            for (int k = 0; k < n; ++k)
+                if (B->m[k]->desc.chains == chains)
+                    for (int c = 0; c < B->m[k]->g.N; c += kTileSizes[s]) *t++ = make_int2(k, c);
+            if (chains) P.nchain[s] = (int)(t - first);
+        }
+        P.tiles[s] = (const int2*)(A + o_tiles[s]);
+    }
+    std::memcpy(image.get() + o_roff, roff.data(), sizeof(int) * (n + 1));
+    std::memset(image.get() + o_rec, 0, L.bytes - o_rec);
     P.descs = (SbBubbleDesc* const*)(A + o_desc);
     P.nb = n;
-    for (int s = 0; s < 3; ++s) {
-        P.tiles[s] = (const int2*)(A + o_tiles[s]);
-        P.ntiles[s] = (int)tiles[s].size();
-    }
     for (int st = 0; st < STAGE_COUNT; ++st) P.sel[st] = 1;
     P.one = nullptr;
     SbSolveSet& S = P.set;
@@ -1667,7 +1668,7 @@ int sb_batch_create(sb_bubble* const* bubbles, int n, sb_batch** out) {
     for (sb_bubble* b : B->m)
         if (e == cudaSuccess) e = cudaMemsetAsync(&b->f.self->halted, 0, sizeof(int), B->stream);
     if (e == cudaSuccess)
-        e = cudaMemcpyAsync(A, image.data(), image.size(), cudaMemcpyHostToDevice, B->stream);
+        e = cudaMemcpyAsync(A, image.get(), L.bytes, cudaMemcpyHostToDevice, B->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(B->stream);
     if (e != cudaSuccess) {
         int r = cuda_fail(e, "sb_batch_create upload");
